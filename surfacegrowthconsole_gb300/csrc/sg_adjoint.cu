@@ -18,13 +18,14 @@
 // The adjoint kernel recomputes rho_i and g_i (first pass over the neighbours) and then adds
 // these terms (second pass): nothing per pair is stored.
 //
-// Pair arithmetic in FP32 (FMA on), per-block parameter sums in shared-memory FP32 (a few
-// thousand terms per block), energies, losses and gradients summed in FP64 across blocks.
+// Pair arithmetic in FP32 (FMA on), parameter sums in FP32 per thread (a few tens of terms) and
+// block, energies, losses and gradients summed in FP64 across blocks.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <string>
 #include <vector>
 
 #include "sg_api.h"
@@ -40,25 +41,41 @@ constexpr int kSI = SG_DIFF_SPLINE_INTERVALS;
 constexpr int kPhi = 2, kDen = 2 + kSC;  // offsets of the two splines in theta
 static_assert(kSC == kSI + 3 && kDP == 2 + 2 * kSC, "spline layout");
 
-struct Spline {
-  float r0, invH;  // first knot, 1 / interval width
-};
+constexpr int kDT = 128;    // threads per block but for the passes over work lists
+// The passes over work lists: warps per slice of 32 atoms, and pairs a thread loads together (a bulk
+// metal atom has 42 to 48, 6 a thread), with what it gathers for them fewer for the sake of registers:
+// 64, four blocks an SM.  Over 64 frames of 20,432 atoms a force-matching evaluation takes 202 us with
+// 8 warps and 3 pairs (6 pairs: 228), 215 with 4 warps, 242 with 16; over 4 frames of 2,217 atoms 49,
+// 60 and 49.
+constexpr int kParts = 8, kLoads = 6, kGathers = 3, kPassThreads = 32 * kParts, kPassBlocks = 4;
 
-// Interval and B-spline weights at r: values b[], derivatives with respect to r db[].
-__device__ __forceinline__ int bspline(const Spline &s, float r, float (&b)[4], float (&db)[4]) {
-  const float x = (r - s.r0) * s.invH;
-  const int k = max(0, min((int)floorf(x), kSI - 1));
-  const float t = x - (float)k, t2 = t * t, t3 = t2 * t, u = 1.f - t;
-  b[0] = u * u * u * (1.f / 6.f);
-  b[1] = (3.f * t3 - 6.f * t2 + 4.f) * (1.f / 6.f);
-  b[2] = (-3.f * t3 + 3.f * t2 + 3.f * t + 1.f) * (1.f / 6.f);
-  b[3] = t3 * (1.f / 6.f);
-  db[0] = -0.5f * u * u * s.invH;
-  db[1] = (1.5f * t2 - 2.f * t) * s.invH;
-  db[2] = (-1.5f * t2 + t + 0.5f) * s.invH;
-  db[3] = 0.5f * t2 * s.invH;
-  return k;
+// The model of one call: epsilon, sigma and both splines as one cubic per interval, in s = r - knot
+// with knot the interval's first knot rounded to float: the coefficients are theta's, expanded around
+// that float in FP64, and s is an exact difference for any r near the interval, so no rounding of
+// knots or widths enters a value or slope.  In device memory, copied there ahead of the passes: as a
+// kernel parameter of this size, every block's read of it took 5 to 12 us of misses in the constant
+// cache.
+struct DiffModel {
+  float4 phi[kSI], den[kSI];
+  float2 knot[kSI];          // {knot, its interval coordinate t (0 but for its rounding)}
+  float r0, invH;            // first knot, 1 / interval width
+  float eps, sig6, invSig;   // epsilon, sigma^6, 1 / sigma
+  float pad;
+};
+static_assert(sizeof(DiffModel) % 16 == 0, "copied as 16-byte words");
+__device__ __forceinline__ void loadModel(const DiffModel *__restrict__ model, DiffModel &m) {
+  const float4 *src = reinterpret_cast<const float4 *>(model);
+  float4 *dst = reinterpret_cast<float4 *>(&m);
+  for (int q = threadIdx.x; q < (int)(sizeof(DiffModel) / 16); q += blockDim.x) dst[q] = src[q];
+  __syncthreads();
 }
+
+// Interval of r (the end pieces continue past the ends).
+__device__ __forceinline__ int interval(const DiffModel &m, float r) {
+  return max(0, min((int)floorf((r - m.r0) * m.invH), kSI - 1));
+}
+__device__ __forceinline__ float cubic(const float4 &c, float s) { return c.x + s * (c.y + s * (c.z + s * c.w)); }
+__device__ __forceinline__ float slope(const float4 &c, float s) { return c.y + s * (2.f * c.z + 3.f * s * c.w); }
 
 // The reference's embedding function (SurfaceGrowth.cu:72-126 forms) with its first and second
 // derivatives.
@@ -82,281 +99,628 @@ __device__ __forceinline__ void embedAll(const RepConst &P, float rho, float &F,
   }
 }
 
-__device__ __forceinline__ float spl(const float *c, int k, const float (&w)[4]) {
-  return c[k] * w[0] + c[k + 1] * w[1] + c[k + 2] * w[2] + c[k + 3] * w[3];
-}
-
-// Block-wide parameter accumulator: shared FP32, flushed into the FP64 totals.
-__device__ __forceinline__ void flushGrad(const float *sG, double *grad) {
-  __syncthreads();
-  for (int q = threadIdx.x; q < kDP; q += blockDim.x)
-    if (sG[q] != 0.f) atomicAdd(&grad[q], (double)sG[q]);
-}
-
+// The sums of an evaluation, the 66 parameters' and the loss, in kSumCopies copies that blocks add
+// to in turn (the host adds the copies): FP64 additions to one address follow one another at about
+// 20 ns, and 912 blocks on one copy ended in 20 us of them.
+constexpr int kSumCopies = 32, kSumStride = kDP + 1, kSums = kSumCopies * kSumStride;
+__device__ __forceinline__ double *sumsCopy(double *sums) { return sums + kSumStride * (blockIdx.x % kSumCopies); }
 __device__ __forceinline__ float warpSumF(float x) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
   return x;
 }
+// ---- pair lists ----------------------------------------------------------------------------
+// Positions are set once for many evaluations of a fit, so everything that follows from them alone
+// is laid out then: which pairs an evaluation needs (a metal atom's metal entries within the EAM
+// cutoff and its carbon entries within the LJ cutoff, and those of the few carbon atoms that have
+// metal within it, out of rows built to the larger cutoff over every species) and each pair's
+// distance and direction, in the order the passes read them.  An evaluation streams
+// them and gathers only what depends on theta.  Before, every pass gathered positions and derived
+// distances anew (about 75 instructions a pair), and a thread per carbon atom walked its whole row
+// (195 us of the 733 us of kernels of a force-matching evaluation over 64 frames of 20,432 atoms).
+//
+// The work lists go in slices of 32 atoms, a lane each, and a slice's pairs are interleaved: pair j
+// of lane l at first + 32 j + l, so that a warp's load of its atoms' j-th pairs is one contiguous
+// piece.  (With 4 to 16 lanes an atom, whose pairs lay in a row, the same passes took 2 to 3 times
+// as long: shorter loops with more remainders, the embedding function for 2 to 8 atoms a warp, and
+// three waves of blocks, each a chain of dependent loads.)
+//
+// Per-atom values are kept in slots: positions in the cell order the list build sorts the atoms
+// into.  The atoms of a warp then share most of their neighbours, and a gather touches few cache
+// lines (metal atoms are numbered by distance from their cluster's centre, which scatters them).
 
-// ---- forward -----------------------------------------------------------------------------
-// Density of every metal atom -> F'(rho) stored; F(rho) added to the frame energy.  kMT lanes
-// per metal atom (kMetalPerBlock atoms per 128-thread block).
-__global__ void __launch_bounds__(128) k_diff_rho(BlockTab tab, const RepConst *__restrict__ rc,
-                                                  const float4 *__restrict__ pos, const int *__restrict__ nn,
-                                                  const int *__restrict__ nbl, int rowStride,
-                                                  const float *__restrict__ theta, Spline sp,
-                                                  float *__restrict__ Fp, double *__restrict__ energy) {
-  __shared__ float sT[kDP];
-  for (int q = threadIdx.x; q < kDP; q += blockDim.x) sT[q] = theta[q];
-  __syncthreads();
-  const int rep = tab.rep[blockIdx.x];
-  const RepConst &P = rc[rep];
-  const int sub = threadIdx.x & (kMT - 1);
-  const unsigned gmask = ((1u << kMT) - 1) << (threadIdx.x & 31 & ~(kMT - 1));
-  const int i = tab.start[blockIdx.x] + threadIdx.x / kMT;
-  const int metalEnd = P.atomOff + P.nMolMe;
-  const bool valid = i < metalEnd;
-  float rho = 0.f;
-  if (valid) {
-    const float4 A = pos[i];
-    const int *row = nbl + (size_t)i * rowStride;
-    for (int j = sub; j < nn[i]; j += kMT) {
-      const int k = row[j];
-      if (k >= metalEnd) continue;
-      const float4 B = pos[k];
-      const float dx = minImg(A.x - B.x, P.region[0]), dy = minImg(A.y - B.y, P.region[1]),
-                  dz = minImg(A.z - B.z, P.region[2]);
-      const float rr = dx * dx + dy * dy + dz * dz;
-      if (rr >= P.rrCutEam) continue;
-      float b[4], db[4];
-      const int kk = bspline(sp, sqrtf(rr), b, db);
-      rho += spl(sT + kDen, kk, b);
-    }
-  }
-#pragma unroll
-  for (int o = kMT / 2; o > 0; o >>= 1) rho += __shfl_xor_sync(gmask, rho, o);
-  float Fv = 0.f;
-  if (valid && sub == 0) {
-    float F, Fd, Fdd;
-    embedAll(P, rho, F, Fd, Fdd);
-    Fp[i] = Fd;
-    Fv = F;
-  }
-  Fv = warpSumF(Fv);
-  if ((threadIdx.x & 31) == 0 && Fv != 0.f) atomicAdd(&energy[rep], (double)Fv);
+// slotOf[atom] (-1: outside the grid, or no lists yet; such an atom has no pair).
+__global__ void k_diff_slots(BlockTab tab, const RepConst *__restrict__ rc, const int *__restrict__ cellStart,
+                             const int *__restrict__ sortIdx, int *__restrict__ slotOf) {
+  const RepConst &P = rc[tab.rep[blockIdx.x]];
+  const int s = tab.start[blockIdx.x] + threadIdx.x;
+  if (s < cellStart[P.cellOff + P.ncells]) slotOf[sortIdx[s]] = s;
 }
-
-// Forces on metal atoms (EAM + LJ with carbon neighbours), pair energies, and with grad != NULL
-// dE/dtheta.
-__global__ void __launch_bounds__(128) k_diff_force_metal(BlockTab tab, const RepConst *__restrict__ rc,
-                                                          const float4 *__restrict__ pos,
-                                                          const int *__restrict__ nn, const int *__restrict__ nbl,
-                                                          int rowStride, const float *__restrict__ theta,
-                                                          Spline sp, const float *__restrict__ Fp,
-                                                          float4 *__restrict__ force, double *__restrict__ energy,
-                                                          double *__restrict__ grad) {
-  __shared__ float sT[kDP], sG[kDP];
-  for (int q = threadIdx.x; q < kDP; q += blockDim.x) {
-    sT[q] = theta[q];
-    sG[q] = 0.f;
-  }
-  __syncthreads();
-  const int rep = tab.rep[blockIdx.x];
-  const RepConst &P = rc[rep];
-  const int sub = threadIdx.x & (kMT - 1);
-  const unsigned gmask = ((1u << kMT) - 1) << (threadIdx.x & 31 & ~(kMT - 1));
-  const int i = tab.start[blockIdx.x] + threadIdx.x / kMT;
-  const int metalEnd = P.atomOff + P.nMolMe;
-  const bool valid = i < metalEnd;
-  const float eps = sT[0], sig = sT[1];
-  float fx = 0.f, fy = 0.f, fz = 0.f, u = 0.f;
-  if (valid) {
-    const float4 A = pos[i];
-    const float Fpi = Fp[i];
-    const int *row = nbl + (size_t)i * rowStride;
-    for (int j = sub; j < nn[i]; j += kMT) {
-      const int k = row[j];
-      const float4 B = pos[k];
-      const float dx = minImg(A.x - B.x, P.region[0]), dy = minImg(A.y - B.y, P.region[1]),
-                  dz = minImg(A.z - B.z, P.region[2]);
-      const float rr = dx * dx + dy * dy + dz * dz;
-      if (k < metalEnd) {
-        if (rr >= P.rrCutEam) continue;
-        const float r = sqrtf(rr);
-        float b[4], db[4];
-        const int kk = bspline(sp, r, b, db);
-        const float phi = spl(sT + kPhi, kk, b), dphi = spl(sT + kPhi, kk, db), df = spl(sT + kDen, kk, db);
-        const float fc = -(dphi + df * (Fpi + Fp[k])) / r;
-        fx += fc * dx; fy += fc * dy; fz += fc * dz;
-        u += 0.5f * phi;
-        if (grad) {
-#pragma unroll
-          for (int m = 0; m < 4; m++) {
-            atomicAdd(&sG[kPhi + kk + m], 0.5f * b[m]);
-            atomicAdd(&sG[kDen + kk + m], Fpi * b[m]);
-          }
-        }
-      } else {
-        if (rr >= P.rrCutLJ) continue;
-        const float s2 = sig * sig / rr, s6 = s2 * s2 * s2, s12 = s6 * s6;
-        const float fc = 24.f * eps * (2.f * s12 - s6) / rr;  // -U'(r) / r
-        fx += fc * dx; fy += fc * dy; fz += fc * dz;
-        u += 4.f * eps * (s12 - s6);                          // the whole pair, from the metal side
-        if (grad) {
-          atomicAdd(&sG[0], 4.f * (s12 - s6));                 // dU / d eps
-          atomicAdd(&sG[1], 24.f * eps * (2.f * s12 - s6) / sig);  // dU / d sigma
-        }
-      }
-    }
-  }
-#pragma unroll
-  for (int o = kMT / 2; o > 0; o >>= 1) {
-    fx += __shfl_xor_sync(gmask, fx, o);
-    fy += __shfl_xor_sync(gmask, fy, o);
-    fz += __shfl_xor_sync(gmask, fz, o);
-    u += __shfl_xor_sync(gmask, u, o);
-  }
-  if (valid && sub == 0) force[i] = make_float4(fx, fy, fz, 0.f);
-  float uw = (sub == 0 && valid) ? u : 0.f;
-  uw = warpSumF(uw);
-  if ((threadIdx.x & 31) == 0 && uw != 0.f) atomicAdd(&energy[rep], (double)uw);
-  if (grad) flushGrad(sG, grad);
-}
-
-// Forces on carbon atoms: LJ with their metal neighbours (their energy is counted on the metal
-// side).  One thread per carbon atom.
-__global__ void __launch_bounds__(128, 8) k_diff_force_carbon(BlockTab tab, const RepConst *__restrict__ rc,
-                                                           const float4 *__restrict__ pos,
-                                                           const int *__restrict__ nn,
-                                                           const int *__restrict__ nbl, int rowStride,
-                                                           const float *__restrict__ theta,
-                                                           float4 *__restrict__ force) {
-  const int rep = tab.rep[blockIdx.x];
-  const RepConst &P = rc[rep];
-  const int i = tab.start[blockIdx.x] + threadIdx.x;
-  if (i >= P.atomOff + P.nMol) return;
-  const int metalEnd = P.atomOff + P.nMolMe;
-  const float eps = theta[0], sig = theta[1];
+// A warp per atom: its row packed to metal entries of higher slots, the other metal entries and
+// carbon entries, with their numbers in seg[slot] (all metal, carbon, metal of higher slots);
+// paired[atom] set for every metal atom in the grid and for a carbon atom of any LJ pair.
+__global__ void __launch_bounds__(kDT) k_diff_pack(BlockTab tab, const RepConst *__restrict__ rc,
+                                                   const float4 *__restrict__ pos, const int *__restrict__ nn,
+                                                   const int *__restrict__ slotOf, int *__restrict__ nbl, int rowStride,
+                                                   int4 *__restrict__ seg, unsigned char *__restrict__ paired) {
+  extern __shared__ int sRow[];
+  const unsigned full = 0xffffffffu;
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int per = 128 / (blockDim.x / 32);  // blocks per table entry (128 atoms)
+  const RepConst &P = rc[tab.rep[blockIdx.x / per]];
+  const int i = tab.start[blockIdx.x / per] + (blockIdx.x % per) * (blockDim.x / 32) + w;
+  if (i >= P.atomOff + P.nMol || slotOf[i] < 0) return;
+  const int metalEnd = P.atomOff + P.nMolMe, own = slotOf[i];
+  const bool metal = i < metalEnd;
+  // what does not go to the front of the row: lower metal entries from the start, carbon from the
+  // end (backwards); together at most the row
+  int *rest = sRow + w * rowStride;
   const float4 A = pos[i];
-  const int *row = nbl + (size_t)i * rowStride;
-  float fx = 0.f, fy = 0.f, fz = 0.f;
-  for (int j = 0; j < nn[i]; j++) {
+  int *row = nbl + (size_t)i * rowStride;
+  const int len = nn[i];
+  int nh = 0, nl = 0, nc = 0;
+  for (int base = 0; base < len; base += 32) {
+    const int k = base + lane < len ? row[base + lane] : -1;
+    bool e = false, c = false;
+    int slot = 0;
+    if (k >= 0 && (metal || k < metalEnd)) {
+      const float4 B = pos[k];
+      const float dx = minImg(A.x - B.x, P.region[0]), dy = minImg(A.y - B.y, P.region[1]),
+                  dz = minImg(A.z - B.z, P.region[2]);
+      const float rr = dx * dx + dy * dy + dz * dz;
+      if (metal && k < metalEnd) e = rr < P.rrCutEam;
+      else c = rr < P.rrCutLJ;
+      if (c) paired[metal ? k : i] = 1;  // seen from either side
+      slot = slotOf[k];
+    }
+    const unsigned lower = (1u << lane) - 1u;
+    const unsigned bh = __ballot_sync(full, e && slot > own), bl = __ballot_sync(full, e && slot < own),
+                   bc = __ballot_sync(full, c);
+    // every lane has read its entry of this and all earlier words: the packed row ends before them
+    if (e && slot > own) row[nh + __popc(bh & lower)] = slot;
+    else if (e) rest[nl + __popc(bl & lower)] = slot;
+    else if (c) rest[rowStride - 1 - nc - __popc(bc & lower)] = slot;
+    nh += __popc(bh);
+    nl += __popc(bl);
+    nc += __popc(bc);
+    __syncwarp();
+  }
+  for (int q = lane; q < nl; q += 32) row[nh + q] = rest[q];
+  for (int q = lane; q < nc; q += 32) row[nh + nl + q] = rest[rowStride - 1 - q];
+  if (lane == 0) {
+    seg[own] = make_int4(nh + nl, nc, nh, 0);
+    if (metal) paired[i] = 1;
+  }
+}
+// An atom of a work list: its slot (-1: a metal atom outside the grid, which has no pair but still
+// its F(0); or none, filling the last slice), its frame (-1: none), its numbers of metal pairs and
+// of carbon pairs after them; the first nh, those with metal atoms of higher slots, are the metal
+// pairs counted once.
+struct DiffWork {
+  int slot, rep, ne, nc, nh, pad[3];
+};
+static_assert(sizeof(DiffWork) == 32, "read in 16-byte words");
+// Appends the lanes with `on` to a work list in lane order.
+__device__ __forceinline__ void appendWork(bool on, int slot, int rep, const int4 *__restrict__ seg,
+                                           DiffWork *__restrict__ list, int *__restrict__ count) {
+  const unsigned full = 0xffffffffu, b = __ballot_sync(full, on);
+  const int lane = threadIdx.x & 31;
+  int at = 0;
+  if (lane == 0 && b) at = atomicAdd(count, __popc(b));
+  at = __shfl_sync(full, at, 0) + __popc(b & ((1u << lane) - 1u));
+  if (!on) return;
+  const int4 c = slot >= 0 ? seg[slot] : make_int4(0, 0, 0, 0);
+  list[at] = DiffWork{slot, rep, c.x, c.y, c.z};
+}
+// The work lists: metal atoms, and carbon atoms with an LJ pair (counts[0], counts[1]).
+__global__ void k_diff_lists(BlockTab tab, const RepConst *__restrict__ rc, const int *__restrict__ cellStart,
+                             const int *__restrict__ sortIdx, const int *__restrict__ slotOf, bool built,
+                             const unsigned char *__restrict__ paired, const int4 *__restrict__ seg,
+                             DiffWork *__restrict__ metal, DiffWork *__restrict__ carbon, int *__restrict__ counts) {
+  const int rep = tab.rep[blockIdx.x], s = tab.start[blockIdx.x] + threadIdx.x;
+  const RepConst &P = rc[rep];
+  const int metalEnd = P.atomOff + P.nMolMe;
+  const int atom = built && s < cellStart[P.cellOff + P.ncells] ? sortIdx[s] : -1;
+  appendWork(atom >= 0 && atom < metalEnd, s, rep, seg, metal, &counts[0]);
+  appendWork(s < metalEnd && slotOf[s] < 0, -1, rep, seg, metal, &counts[0]);
+  appendWork(atom >= metalEnd && paired[atom], s, rep, seg, carbon, &counts[1]);
+}
+
+// A slice of 32 atoms of a work list: where its pairs start, the most metal and carbon pairs of an
+// atom (an atom's carbon pairs follow the most metal ones), and where its metal pairs counted once do.
+struct DiffSlice {
+  int first, most, mostC, once;
+};
+// A warp per slice; totals: places taken by the pairs of all slices, metal pairs counted once.  The
+// last slice is filled.
+__global__ void __launch_bounds__(kDT) k_diff_slices(DiffWork *__restrict__ list, int n, DiffSlice *__restrict__ slices,
+                                                     unsigned long long *__restrict__ totals) {
+  const unsigned full = 0xffffffffu;
+  const int s = blockIdx.x * (kDT / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31, u = 32 * s + lane;
+  if (32 * s >= n) return;
+  DiffWork w{-1, -1, 0, 0, 0};
+  if (u < n) w = list[u];
+  else list[u] = w;
+  const int most = __reduce_max_sync(full, w.ne), mostC = __reduce_max_sync(full, w.nc), once = __reduce_add_sync(full, w.nh);
+  if (lane == 0)
+    slices[s] = DiffSlice{(int)atomicAdd(&totals[0], 32ull * (most + mostC)), most, mostC,
+                          (int)atomicAdd(&totals[1], (unsigned long long)once)};
+}
+
+// Pairs as the passes read them: the other atom's slot, the distance, and the direction (from the
+// other atom to this one).
+struct DiffPairs {
+  int *slot;
+  float *r;
+  float4 *dir;  // w: the distance again
+  float *w;     // of an evaluation
+  int2 *both;   // the metal pairs counted once: both slots, the distance, the place of its w
+  float *rOnce;
+  int *place;
+};
+// A warp per atom of a work list.
+__global__ void __launch_bounds__(kDT) k_diff_pairs(const DiffWork *__restrict__ list, const DiffSlice *__restrict__ slices,
+                                                    int n, const RepConst *__restrict__ rc,
+                                                    const float4 *__restrict__ slotPos, const int *__restrict__ nbl,
+                                                    int rowStride, DiffPairs pr) {
+  const int u = blockIdx.x * (kDT / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (u >= n || list[u].slot < 0) return;
+  const DiffWork a = list[u];
+  const DiffSlice sl = slices[u / 32];
+  const RepConst &P = rc[a.rep];
+  const float4 A = slotPos[a.slot];
+  const int *row = nbl + (size_t)__float_as_int(A.w) * rowStride;
+  for (int j = lane; j < a.ne + a.nc; j += 32) {
     const int k = row[j];
-    if (k >= metalEnd) continue;
-    const float4 B = pos[k];
+    const float4 B = slotPos[k];
     const float dx = minImg(A.x - B.x, P.region[0]), dy = minImg(A.y - B.y, P.region[1]),
                 dz = minImg(A.z - B.z, P.region[2]);
-    const float rr = dx * dx + dy * dy + dz * dz;
-    if (rr >= P.rrCutLJ) continue;
-    const float s2 = sig * sig / rr, s6 = s2 * s2 * s2, s12 = s6 * s6;
-    const float fc = 24.f * eps * (2.f * s12 - s6) / rr;
-    fx += fc * dx; fy += fc * dy; fz += fc * dz;
+    const float r = sqrtf(dx * dx + dy * dy + dz * dz);
+    const int at = sl.first + 32 * (j < a.ne ? j : sl.most + j - a.ne) + u % 32;
+    pr.slot[at] = k;
+    pr.r[at] = r;
+    pr.dir[at] = make_float4(dx / r, dy / r, dz / r, r);
   }
-  force[i] = make_float4(fx, fy, fz, 0.f);
 }
-
-// ---- force matching ------------------------------------------------------------------------
-// Residual e_i = scale (F_i - F_ref,i) into resid (which holds F_ref on entry) and the loss sum
-// |F_i - F_ref,i|^2 (times lossScale) into loss.
-__global__ void k_diff_resid(int n, const float4 *__restrict__ force, float4 *__restrict__ resid, float scale,
-                             double lossScale, double *__restrict__ loss) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  float s = 0.f;
-  if (i < n) {
-    const float4 f = force[i], ref = resid[i];
-    const float ex = f.x - ref.x, ey = f.y - ref.y, ez = f.z - ref.z;
-    s = ex * ex + ey * ey + ez * ez;
-    resid[i] = make_float4(scale * ex, scale * ey, scale * ez, 0.f);
-  }
-  s = warpSumF(s);
-  if ((threadIdx.x & 31) == 0 && s != 0.f) atomicAdd(loss, lossScale * (double)s);
-}
-
-// Adjoint of the force-matching loss over the metal atoms' pairs (every metal-metal pair from
-// both sides, every metal-carbon pair from its metal side): dD/dtheta into grad (dL/dtheta is
-// its negative).  First pass: rho_i and g_i recomputed; second pass: the gradient terms.
-__global__ void __launch_bounds__(128) k_diff_adjoint(BlockTab tab, const RepConst *__restrict__ rc,
-                                                      const float4 *__restrict__ pos,
-                                                      const int *__restrict__ nn, const int *__restrict__ nbl,
-                                                      int rowStride, const float *__restrict__ theta, Spline sp,
-                                                      const float4 *__restrict__ resid, double *__restrict__ grad) {
-  __shared__ float sT[kDP], sG[kDP];
-  for (int q = threadIdx.x; q < kDP; q += blockDim.x) {
-    sT[q] = theta[q];
-    sG[q] = 0.f;
-  }
-  __syncthreads();
-  const int rep = tab.rep[blockIdx.x];
-  const RepConst &P = rc[rep];
-  const int sub = threadIdx.x & (kMT - 1);
-  const unsigned gmask = ((1u << kMT) - 1) << (threadIdx.x & 31 & ~(kMT - 1));
-  const int i = tab.start[blockIdx.x] + threadIdx.x / kMT;
-  const int metalEnd = P.atomOff + P.nMolMe;
-  const bool valid = i < metalEnd;
-  const float eps = sT[0], sig = sT[1];
-  float4 A = make_float4(0.f, 0.f, 0.f, 0.f), Ei = A;
-  const int *row = nbl + (size_t)i * rowStride;
-  const int n = valid ? nn[i] : 0;
-  float rho = 0.f, g = 0.f;
-  if (valid) {
-    A = pos[i];
-    Ei = resid[i];
-    for (int j = sub; j < n; j += kMT) {
-      const int k = row[j];
-      if (k >= metalEnd) continue;
-      const float4 B = pos[k];
-      const float dx = minImg(A.x - B.x, P.region[0]), dy = minImg(A.y - B.y, P.region[1]),
-                  dz = minImg(A.z - B.z, P.region[2]);
-      const float rr = dx * dx + dy * dy + dz * dz;
-      if (rr >= P.rrCutEam) continue;
-      const float r = sqrtf(rr);
-      float b[4], db[4];
-      const int kk = bspline(sp, r, b, db);
-      const float4 Ek = resid[k];
-      const float w = (dx * (Ei.x - Ek.x) + dy * (Ei.y - Ek.y) + dz * (Ei.z - Ek.z)) / r;
-      rho += spl(sT + kDen, kk, b);
-      g += spl(sT + kDen, kk, db) * w;
+// A warp per slice: its metal pairs counted once, in the order of their places, so that what is read
+// at the places of neighbouring ones lies together.
+__global__ void __launch_bounds__(kDT) k_diff_once(const DiffWork *__restrict__ list, const DiffSlice *__restrict__ slices,
+                                                   int n, DiffPairs pr) {
+  const int s = blockIdx.x * (kDT / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (32 * s >= n) return;
+  const DiffWork a = list[32 * s + lane];
+  const DiffSlice sl = slices[s];
+  int at = sl.once;
+  for (int j = 0; j < sl.most; j++) {
+    const unsigned b = __ballot_sync(0xffffffffu, j < a.nh);
+    if (j < a.nh) {
+      const int place = sl.first + 32 * j + lane, q = at + __popc(b & ((1u << lane) - 1u));
+      pr.both[q] = make_int2(a.slot, pr.slot[place]);
+      pr.rOnce[q] = pr.r[place];
+      pr.place[q] = place;
     }
+    at += __popc(b);
   }
+}
+
+// ---- evaluation ----------------------------------------------------------------------------
+// All passes over work lists: a lane per atom, a slice a block at a time, kParts warps that take every
+// kParts-th pair each; their sums meet in shared memory.  A load that misses L1 takes 0.5 us here, and
+// what a pass costs is the number of such loads that wait for one another: a thread loads several pairs
+// together, and the next slice's work entries while this one is evaluated.  A block walks the slices
+// with a grid stride, so that it loads the model once.
+struct DiffAtom {
+  int slot, rep, ne, nc, nh;  // as DiffWork; slot -1, no pairs and rep -1 past the end of the list
+  int first, most, mostC;           // as DiffSlice
+};
+__device__ __forceinline__ DiffAtom diffAtom(const DiffWork *__restrict__ list, const DiffSlice *__restrict__ slices, int n,
+                                             int slice) {
+  if (32 * slice >= n) return DiffAtom{-1, -1, 0, 0, 0, 0, 0, 0};
+  const DiffWork *w = list + 32 * slice + (threadIdx.x & 31);
+  const int4 w0 = *reinterpret_cast<const int4 *>(w), s = *reinterpret_cast<const int4 *>(slices + slice);
+  return DiffAtom{w0.x, w0.y, w0.z, w0.w, w->nh, s.x, s.y, s.z};
+}
+// Sums of x over the parts, for part 0 (warp 0).  Two buffers in turn: the others may write the next
+// slice's while part 0 still reads this one's.
+template <int N>
+__device__ __forceinline__ void sumParts(int turn, float (&x)[N]) {
+  __shared__ float s[2][kParts][N][32];
+  const int part = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll
-  for (int o = kMT / 2; o > 0; o >>= 1) {
-    rho += __shfl_xor_sync(gmask, rho, o);
-    g += __shfl_xor_sync(gmask, g, o);
+  for (int k = 0; k < N; k++) s[turn & 1][part][k][lane] = x[k];
+  __syncthreads();
+  if (part != 0) return;
+#pragma unroll
+  for (int k = 0; k < N; k++) {
+    x[k] = 0.f;
+#pragma unroll
+    for (int p = 0; p < kParts; p++) x[k] += s[turn & 1][p][k][lane];
   }
-  if (valid) {
-    float F, Fd, Fdd;
-    embedAll(P, rho, F, Fd, Fdd);
-    const float gF = Fdd * g;
-    for (int j = sub; j < n; j += kMT) {
-      const int k = row[j];
-      const float4 B = pos[k];
-      const float dx = minImg(A.x - B.x, P.region[0]), dy = minImg(A.y - B.y, P.region[1]),
-                  dz = minImg(A.z - B.z, P.region[2]);
-      const float rr = dx * dx + dy * dy + dz * dz;
-      const float4 Ek = resid[k];
-      const float de = dx * (Ei.x - Ek.x) + dy * (Ei.y - Ek.y) + dz * (Ei.z - Ek.z);
-      if (k < metalEnd) {
-        if (rr >= P.rrCutEam) continue;
-        const float r = sqrtf(rr), w = de / r;
-        float b[4], db[4];
-        const int kk = bspline(sp, r, b, db);
+}
+// f(u, j) over a thread's share of its atom's n pairs j (at first + 32 j + lane), the most of any lane
+// of the slice being `most`; U at a time, load(u, place) for all of them first.
+template <int U, typename Load, typename F>
+__device__ __forceinline__ void overPairs(int first, int n, int most, Load load, F f) {
+  const int lane = threadIdx.x & 31;
+  for (int j0 = threadIdx.x >> 5; j0 < most; j0 += U * kParts) {
 #pragma unroll
-        for (int m = 0; m < 4; m++) {
-          atomicAdd(&sG[kPhi + kk + m], 0.5f * db[m] * w);
-          atomicAdd(&sG[kDen + kk + m], gF * b[m] + Fd * db[m] * w);
-        }
-      } else {
-        if (rr >= P.rrCutLJ) continue;
-        const float r = sqrtf(rr), w = de / r;
-        const float s2 = sig * sig / rr, s6 = s2 * s2 * s2, s12 = s6 * s6;
-        atomicAdd(&sG[0], 24.f * (s6 - 2.f * s12) / r * w);                    // dU'/d eps
-        atomicAdd(&sG[1], 144.f * eps * (s6 - 4.f * s12) / (r * sig) * w);     // dU'/d sigma
+    for (int u = 0; u < U; u++)
+      if (j0 + u * kParts < n) load(u, first + 32 * (j0 + u * kParts) + lane);
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (j0 + u * kParts < n) f(u, j0 + u * kParts);
+  }
+}
+// (sigma / r)^6 of an LJ pair
+__device__ __forceinline__ float ljSix(float sig6, float r) {
+  const float i2 = 1.f / (r * r);
+  return sig6 * (i2 * i2 * i2);
+}
+
+// Densities: F'(rho) and F''(rho) of every metal atom (emb, by slot); with ENERGY also the frame
+// energies (to which it only adds), else the launch clears the sums of the evaluation (sums), and
+// its first refBlocks blocks fetch the reference forces of the atoms with pairs (into refOf, by slot)
+// for the force pass, which a read over the host link by each of its atoms would hold up.
+template <bool ENERGY>
+__global__ void __launch_bounds__(kPassThreads) k_diff_rho(const DiffModel *__restrict__ model, const DiffWork *__restrict__ metal,
+                                                  const DiffSlice *__restrict__ slices, int nMetal,
+                                                  const RepConst *__restrict__ rc, const float *__restrict__ pairR,
+                                                  float2 *__restrict__ emb, double *__restrict__ energy,
+                                                  double *__restrict__ sums, const float *__restrict__ ref, int n,
+                                                  const unsigned char *__restrict__ paired, const int *__restrict__ slotOf,
+                                                  float4 *__restrict__ refOf, int refBlocks) {
+  __shared__ __align__(16) DiffModel m;
+  pdlEnter();
+  if (!ENERGY && blockIdx.x == 0)
+    for (int q = threadIdx.x; q < kSums; q += blockDim.x) sums[q] = 0.0;
+  const int block = (int)blockIdx.x - refBlocks;
+  if (!ENERGY && block < 0) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += refBlocks * blockDim.x)
+      if (paired[i]) refOf[slotOf[i]] = make_float4(ref[3 * (size_t)i], ref[3 * (size_t)i + 1], ref[3 * (size_t)i + 2], 0.f);
+    return;
+  }
+  const int grid = gridDim.x - refBlocks, nSlices = (nMetal + 31) / 32, lane = threadIdx.x & 31;
+  DiffAtom next = diffAtom(metal, slices, nMetal, block);
+  loadModel(model, m);
+  for (int slice = block, turn = 0; slice < nSlices; slice += grid, turn++) {
+    const DiffAtom a = next;
+    next = diffAtom(metal, slices, nMetal, slice + grid);
+    float x[2] = {0.f, 0.f};  // rho, pair energy
+    float r[kLoads];
+    auto load = [&](int u, int p) { r[u] = pairR[p]; };
+    overPairs<kLoads>(a.first, a.ne, a.most, load, [&](int u, int) {
+      const int i = interval(m, r[u]);
+      const float s = r[u] - m.knot[i].x;
+      x[0] += cubic(m.den[i], s);
+      if (ENERGY) x[1] += 0.5f * cubic(m.phi[i], s);
+    });
+    if (ENERGY)
+      overPairs<kLoads>(a.first + 32 * a.most, a.nc, a.mostC, load, [&](int u, int) {
+        const float s6 = ljSix(m.sig6, r[u]);
+        x[1] += 4.f * m.eps * (s6 * s6 - s6);  // the whole pair, from the metal side
+      });
+    sumParts(turn, x);
+    if (threadIdx.x >= 32) continue;
+    float F = 0.f, Fd, Fdd;
+    if (a.rep >= 0) embedAll(rc[a.rep], x[0], F, Fd, Fdd);
+    if (a.slot >= 0) emb[a.slot] = make_float2(Fd, Fdd);
+    if (ENERGY) {
+      // the slice's atoms of one frame in one sum; a slice whose atoms are of several adds them singly
+      const int rep = __shfl_sync(0xffffffffu, a.rep, 0);
+      if (__all_sync(0xffffffffu, a.rep < 0 || a.rep == rep)) {
+        const float u = warpSumF(x[1]), Fw = warpSumF(F);
+        if (lane == 0 && rep >= 0) atomicAdd(&energy[rep], (double)u + (double)Fw);
+      } else if (a.rep >= 0) {
+        atomicAdd(&energy[a.rep], (double)x[1] + (double)F);
       }
     }
   }
-  flushGrad(sG, grad);
 }
+
+// Sum over the block (all threads), in thread 0: FP32 in a warp, FP64 over the warps.  (FP64 runs at
+// 1/64 of the FP32 rate here: with the warps' sums in FP64 too, a block of 8 warps kept the SM's FP64
+// pipe busy for 1,700 cycles, and this sum took half of the force pass.)
+__device__ __forceinline__ double blockSum(float x) {
+  __shared__ float s[32];
+  x = warpSumF(x);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = x;
+  __syncthreads();
+  double y = 0.0;
+  if (threadIdx.x == 0)
+    for (int q = 0; q < (int)blockDim.x / 32; q++) y += (double)s[q];
+  return y;
+}
+
+// |F_ref|^2 summed over the atoms without a pair (their force is zero), for block b of nb: the
+// reference forces stream in place, from host memory where the device reads it directly.
+__device__ __forceinline__ float refSquares(const float *__restrict__ ref, int n, const unsigned char *__restrict__ paired,
+                                            int b, int nb) {
+  const long long n3 = 3LL * n;
+  const bool aligned = (reinterpret_cast<uintptr_t>(ref) & 15) == 0;
+  const long long n4 = aligned ? n3 / 4 : 0, stride = (long long)nb * blockDim.x;
+  float s = 0.f;
+  for (long long q = (long long)b * blockDim.x + threadIdx.x; q < n4; q += 2 * stride) {
+    float4 v[2];
+#pragma unroll
+    for (int u = 0; u < 2; u++)
+      v[u] = q + u * stride < n4 ? reinterpret_cast<const float4 *>(ref)[q + u * stride] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+      // floats f .. f + 3 belong to atoms a and a + 1, split at atom a + 1's first float
+      const long long f = min(4 * (q + u * stride), n3 - 1);
+      const int a = (int)(f / 3), cut = (int)(3LL * (a + 1) - f);  // 1..3 floats of atom a
+      const float wa = paired[a] ? 0.f : 1.f, wb = (a + 1 < n && !paired[a + 1]) ? 1.f : 0.f;
+      s += wa * (v[u].x * v[u].x) + (cut > 1 ? wa : wb) * (v[u].y * v[u].y) + (cut > 2 ? wa : wb) * (v[u].z * v[u].z) +
+           wb * (v[u].w * v[u].w);
+    }
+  }
+  for (long long f = 4 * n4 + (long long)b * blockDim.x + threadIdx.x; f < n3; f += stride)
+    if (!paired[f / 3]) s += ref[f] * ref[f];
+  return s;
+}
+__global__ void __launch_bounds__(kDT) k_diff_ref(const float *__restrict__ ref, int n,
+                                                  const unsigned char *__restrict__ paired, double *__restrict__ lossPart) {
+  const double s = blockSum(refSquares(ref, n, paired, blockIdx.x, gridDim.x));
+  if (threadIdx.x == 0) lossPart[blockIdx.x] = s;
+}
+
+// Forces of the metal atoms (EAM and LJ) and of the paired carbon atoms (LJ), slices of the
+// metal list first.  LOSS: the residual e = scale (F - F_ref) of each (resid, by slot; F_ref on
+// entry) and sum |F - F_ref|^2 (sums), the last refBlocks blocks of the grid summing the atoms without
+// a pair (refPart); else the forces, packed (out).
+template <bool LOSS>
+__global__ void __launch_bounds__(kPassThreads, kPassBlocks) k_diff_force(const DiffModel *__restrict__ model, const DiffWork *__restrict__ metal,
+                                                    const DiffSlice *__restrict__ metalSlices, int nMetal,
+                                                    const DiffWork *__restrict__ carbon,
+                                                    const DiffSlice *__restrict__ carbonSlices, int nCarbon,
+                                                    const int *__restrict__ sortIdx, DiffPairs pr,
+                                                    const float2 *__restrict__ emb, float *__restrict__ out,
+                                                    const float *__restrict__ ref, float scale,
+                                                    float4 *__restrict__ resid, double *__restrict__ sums,
+                                                    double *__restrict__ refPart, int n,
+                                                    const unsigned char *__restrict__ paired, int refBlocks) {
+  __shared__ __align__(16) DiffModel m;
+  pdlEnter();
+  const int grid = gridDim.x - refBlocks;
+  if (LOSS && (int)blockIdx.x >= grid) {
+    const double s = blockSum(refSquares(ref, n, paired, blockIdx.x - grid, refBlocks));
+    if (threadIdx.x == 0) refPart[blockIdx.x - grid] = s;
+    return;
+  }
+  const int metalN = (nMetal + 31) / 32, nSlices = metalN + (nCarbon + 31) / 32;
+  auto atomOf = [&](int slice) {
+    return slice < metalN ? diffAtom(metal, metalSlices, nMetal, slice)
+                          : diffAtom(carbon, carbonSlices, nCarbon, slice - metalN);
+  };
+  DiffAtom next = atomOf(blockIdx.x);
+  loadModel(model, m);
+  float loss = 0.f;
+  for (int slice = blockIdx.x, turn = 0; slice < nSlices; slice += grid, turn++) {
+    const DiffAtom a = next;
+    next = atomOf(slice + grid);
+    float x[3] = {0.f, 0.f, 0.f};
+    const float Fpi = a.ne ? emb[a.slot].x : 0.f;
+    float4 D[kGathers];
+    float Fk[kGathers];
+    overPairs<kGathers>(
+        a.first, a.ne, a.most,
+        [&](int u, int p) {
+          D[u] = pr.dir[p];
+          Fk[u] = emb[pr.slot[p]].x;
+        },
+        [&](int u, int) {
+          const int i = interval(m, D[u].w);
+          const float s = D[u].w - m.knot[i].x;
+          const float f = -(slope(m.phi[i], s) + slope(m.den[i], s) * (Fpi + Fk[u]));
+          x[0] += f * D[u].x; x[1] += f * D[u].y; x[2] += f * D[u].z;
+        });
+    overPairs<kGathers>(
+        a.first + 32 * a.most, a.nc, a.mostC, [&](int u, int p) { D[u] = pr.dir[p]; },
+        [&](int u, int) {
+          const float s6 = ljSix(m.sig6, D[u].w), s12 = s6 * s6;
+          const float f = 24.f * m.eps * (2.f * s12 - s6) / D[u].w;  // -U'(r)
+          x[0] += f * D[u].x; x[1] += f * D[u].y; x[2] += f * D[u].z;
+        });
+    sumParts(turn, x);
+    if (threadIdx.x < 32 && a.slot >= 0) {
+      if (LOSS) {
+        const float4 want = resid[a.slot];
+        const float ex = x[0] - want.x, ey = x[1] - want.y, ez = x[2] - want.z;
+        resid[a.slot] = make_float4(scale * ex, scale * ey, scale * ez, 0.f);
+        loss += ex * ex + ey * ey + ez * ez;
+      } else {
+        const size_t f = 3 * (size_t)sortIdx[a.slot];
+        out[f] = x[0];
+        out[f + 1] = x[1];
+        out[f + 2] = x[2];
+      }
+    }
+  }
+  if (LOSS && threadIdx.x < 32) {
+    loss = warpSumF(loss);
+    if (threadIdx.x == 0) atomicAdd(sumsCopy(sums) + kDP, (double)loss);
+  }
+}
+
+// Parameter sums.  A pair adds to four consecutive coefficients of each spline.  Every thread has
+// a column of its own in shared memory ({phi, f} of coefficient c at [c][thread], 32 KB a block,
+// no bank shared between lanes), so an addition is a plain load and store; a float atomicAdd in
+// shared memory is a compare-and-swap loop whose lanes collide, since neighbours sit at few
+// distances.  The blocks are few and walk many atoms, because each ends with 66 FP64 additions to
+// the same 66 totals: a block per 8 atoms took 16,000 x 66 of them.
+struct DiffSums {
+  float2 c[kSC][kDT];
+};
+// A pair at interval coordinate t of interval k adds p0 b_m + p1 b'_m to phi's coefficient k + m
+// and d0 b_m + d1 b'_m to f's: b, b' the B-spline weights at t and their t-derivatives.
+template <bool VAL, bool DER>
+__device__ __forceinline__ void addPair(DiffSums &S, int k, float t, float p0, float p1, float d0, float d1) {
+  const float u = 1.f - t, t2 = t * t, u2 = u * u;
+  const float b[4] = {u2 * (u * (1.f / 6.f)), fmaf(t2, fmaf(0.5f, t, -1.f), 2.f / 3.f),
+                      fmaf(u2, fmaf(0.5f, u, -1.f), 2.f / 3.f), t2 * (t * (1.f / 6.f))};
+  const float db[4] = {-0.5f * u2, t * fmaf(1.5f, t, -2.f), -u * fmaf(1.5f, u, -2.f), 0.5f * t2};
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    float2 v = S.c[k + q][threadIdx.x];
+    if (VAL) v.x += p0 * b[q];
+    if (DER) v.x += p1 * db[q];
+    v.y += d0 * b[q];
+    if (DER) v.y += d1 * db[q];
+    S.c[k + q][threadIdx.x] = v;
+  }
+}
+__device__ __forceinline__ void clearSums(DiffSums &S) {
+#pragma unroll 8
+  for (int q = 0; q < kSC; q++) S.c[q][threadIdx.x] = make_float2(0.f, 0.f);
+}
+// The block's columns into the totals.
+__device__ __forceinline__ void flushSums(const DiffSums &S, double *__restrict__ grad) {
+  __syncthreads();
+  grad = sumsCopy(grad);
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int q = w; q < kSC; q += kDT / 32) {
+    float px = 0.f, py = 0.f;
+#pragma unroll
+    for (int u = 0; u < kDT / 32; u++) {
+      const float2 v = S.c[q][lane + 32 * u];
+      px += v.x;
+      py += v.y;
+    }
+    px = warpSumF(px);
+    py = warpSumF(py);
+    if (lane == 0) {
+      if (px != 0.f) atomicAdd(&grad[kPhi + q], (double)px);
+      if (py != 0.f) atomicAdd(&grad[kDen + q], (double)py);
+    }
+  }
+}
+
+// The LJ parameters' share of an evaluation's gradient, and with LOSS what the metal pairs' share
+// needs of each atom and pair: {F'(rho_i), F''(rho_i) g_i} (emb) and w (pr.w, pairs counted once).
+template <bool LOSS>
+__global__ void __launch_bounds__(kPassThreads, kPassBlocks) k_diff_along(const DiffModel *__restrict__ model, const DiffWork *__restrict__ metal,
+                                                    const DiffSlice *__restrict__ slices, int nMetal, DiffPairs pr,
+                                                    const float4 *__restrict__ resid, float2 *__restrict__ emb,
+                                                    double *__restrict__ sums) {
+  __shared__ __align__(16) DiffModel m;
+  pdlEnter();
+  const int nSlices = (nMetal + 31) / 32;
+  DiffAtom next = diffAtom(metal, slices, nMetal, blockIdx.x);
+  loadModel(model, m);
+  float ge = 0.f, gs = 0.f;
+  for (int slice = blockIdx.x, turn = 0; slice < nSlices; slice += gridDim.x, turn++) {
+    const DiffAtom a = next;
+    next = diffAtom(metal, slices, nMetal, slice + gridDim.x);
+    if (LOSS) {
+      const float4 Ei = a.slot >= 0 ? resid[a.slot] : make_float4(0.f, 0.f, 0.f, 0.f);
+      const float Fdd = a.slot >= 0 ? emb[a.slot].y : 0.f;
+      float x[1] = {0.f};  // g
+      float4 D[kGathers], E[kGathers];
+      auto load = [&](int u, int p) {
+        D[u] = pr.dir[p];
+        E[u] = resid[pr.slot[p]];
+      };
+      auto along = [&](int u) {  // w = rhat . (e_i - e_k)
+        return D[u].x * (Ei.x - E[u].x) + D[u].y * (Ei.y - E[u].y) + D[u].z * (Ei.z - E[u].z);
+      };
+      overPairs<kGathers>(a.first, a.ne, a.most, load, [&](int u, int j) {
+        const float w = along(u);
+        const int i = interval(m, D[u].w);
+        x[0] += slope(m.den[i], D[u].w - m.knot[i].x) * w;
+        if (j < a.nh) pr.w[a.first + 32 * j + (threadIdx.x & 31)] = w;
+      });
+      overPairs<kGathers>(a.first + 32 * a.most, a.nc, a.mostC, load, [&](int u, int) {
+        const float w = along(u);
+        const float s6 = ljSix(m.sig6, D[u].w), s12 = s6 * s6;
+        ge += 24.f * (s6 - 2.f * s12) / D[u].w * w;                          // dU'/d eps
+        gs += 144.f * m.eps * (s6 - 4.f * s12) / D[u].w * m.invSig * w;  // dU'/d sigma
+      });
+      sumParts(turn, x);
+      if (threadIdx.x < 32 && a.slot >= 0) emb[a.slot].y = Fdd * x[0];
+    } else {
+      float r[kLoads];
+      overPairs<kLoads>(a.first + 32 * a.most, a.nc, a.mostC, [&](int u, int p) { r[u] = pr.r[p]; },
+                       [&](int u, int) {
+                         const float s6 = ljSix(m.sig6, r[u]), s12 = s6 * s6;
+                         ge += 4.f * (s12 - s6);                                // dU / d eps
+                         gs += 24.f * m.eps * (2.f * s12 - s6) * m.invSig;  // dU / d sigma
+                       });
+    }
+  }
+  const double e = blockSum(ge), q = blockSum(gs);
+  if (threadIdx.x == 0 && e != 0.0) atomicAdd(sumsCopy(sums), e);
+  if (threadIdx.x == 0 && q != 0.0) atomicAdd(sumsCopy(sums) + 1, q);
+}
+
+// The spline coefficients' share, a thread per metal pair counted once (its two sides' terms are
+// alike: r and w are the same from both, and only F' and F'' g differ).
+//   energy: phi B(r), f (F'_i + F'_j) B(r)
+//   loss (LOSS; the adjoint of sum e . dE/dr): phi w B'(r), f (F''_i g_i + F''_j g_j) B(r) +
+//   (F'_i + F'_j) w B'(r).
+constexpr int kSumLoads = 4;  // pairs a thread loads together
+template <bool LOSS>
+__global__ void __launch_bounds__(kDT) k_diff_sums(const DiffModel *__restrict__ model, DiffPairs pr, int nPairs,
+                                                   const float2 *__restrict__ emb, double *__restrict__ grad) {
+  __shared__ __align__(16) DiffModel m;
+  __shared__ DiffSums S;
+  clearSums(S);
+  loadModel(model, m);
+  pdlEnter();
+  const int stride = gridDim.x * kDT;
+  for (int p0 = blockIdx.x * kDT + threadIdx.x; p0 < nPairs; p0 += kSumLoads * stride) {
+    float r[kSumLoads], w[kSumLoads];
+    int at[kSumLoads];
+    int2 k[kSumLoads];
+    float2 a[kSumLoads], b[kSumLoads];
+#pragma unroll
+    for (int q = 0; q < kSumLoads; q++) {
+      const int p = p0 + q * stride;
+      if (p < nPairs) {
+        k[q] = pr.both[p];
+        r[q] = pr.rOnce[p];
+        if (LOSS) at[q] = pr.place[p];
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < kSumLoads; q++)
+      if (p0 + q * stride < nPairs) {
+        a[q] = emb[k[q].x];
+        b[q] = emb[k[q].y];
+        if (LOSS) w[q] = pr.w[at[q]];
+      }
+#pragma unroll
+    for (int q = 0; q < kSumLoads; q++) {
+      if (p0 + q * stride >= nPairs) continue;
+      const int i = interval(m, r[q]);
+      const float t = fmaf(r[q] - m.knot[i].x, m.invH, m.knot[i].y), Fd = a[q].x + b[q].x;
+      if (LOSS) {
+        const float wh = w[q] * m.invH;
+        addPair<false, true>(S, i, t, 0.f, wh, a[q].y + b[q].y, Fd * wh);
+      } else {
+        addPair<true, false>(S, i, t, 1.f, 0.f, Fd, 0.f);
+      }
+    }
+  }
+  flushSums(S, grad);
+}
+
+// Most blocks of a pass: those resident at once.  Blocks of a second wave would start when the first
+// has done nearly all the work.
+template <typename K>
+static int mostBlocks(K kernel, int threads, int numSMs) {
+  int n = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, 0) != cudaSuccess || n < 1) n = 1;
+  return n * numSMs;
+}
+struct DiffGrids {
+  int rho, energy, residual, force, along, lj, lossSums, energySums;
+  explicit DiffGrids(int sms)
+      : rho(mostBlocks(k_diff_rho<false>, kPassThreads, sms)), energy(mostBlocks(k_diff_rho<true>, kPassThreads, sms)),
+        residual(mostBlocks(k_diff_force<true>, kPassThreads, sms)), force(mostBlocks(k_diff_force<false>, kPassThreads, sms)),
+        along(mostBlocks(k_diff_along<true>, kPassThreads, sms)), lj(mostBlocks(k_diff_along<false>, kPassThreads, sms)),
+        lossSums(mostBlocks(k_diff_sums<true>, kDT, sms)), energySums(mostBlocks(k_diff_sums<false>, kDT, sms)) {}
+};
 
 }  // namespace sg
 
@@ -365,11 +729,28 @@ using namespace sg;
 struct sg_diff {
   sg_ctx *ctx = nullptr;
   int nFrames = 0, n = 0;
-  Spline sp{};
-  float *theta = nullptr, *Fp = nullptr;
-  float4 *force = nullptr, *resid = nullptr;
-  double *energy = nullptr, *grad = nullptr, *loss = nullptr;
-  sg_simparams p0{};
+  DiffGrids most;
+  explicit sg_diff(int sms) : most(sms) {}
+  double r0 = 0, h = 0;  // first knot and interval width of the splines
+  bool listed = false;                          // has work lists (of positions, or of none yet)
+  void *arena = nullptr, *pairArena = nullptr, *pinned = nullptr;  // what the arrays below lie in
+  int *slotOf = nullptr;                        // slot of each atom
+  unsigned char *paired = nullptr;              // per atom: has a slot in a work list
+  DiffWork *metal = nullptr, *carbon = nullptr;  // the work lists and their slices
+  DiffSlice *metalSlices = nullptr, *carbonSlices = nullptr;
+  int *counts = nullptr, nMetal = 0, nCarbon = 0;
+  unsigned long long *totals = nullptr;         // places of all pairs, metal pairs counted once
+  int4 *seg = nullptr;                          // per slot: its row's segments (k_diff_pack)
+  DiffPairs pairs{};
+  unsigned long long pairCap = 0, onceCap = 0;  // pairs the arrays hold
+  int nOnce = 0;
+  float2 *emb = nullptr;                        // per slot: F', then F'' or F'' g
+  float4 *resid = nullptr;                      // per slot
+  // results on the device and page-locked on the host: the copies of the sums, then the
+  // frame energies or the sums of squares of the blocks of k_diff_ref
+  double *out = nullptr, *hostOut = nullptr;
+  DiffModel *model = nullptr, *hostModel = nullptr;  // of the call, on the device and page-locked
+  int outCap = 0;
 };
 
 #define DCK(call)                                                                              \
@@ -387,9 +768,10 @@ static void eamAnalytic(const sg_simparams &p, double r, double &phi, double &f)
   f = p.fe * eB / dB;
 }
 
-static Spline splineOf(const sg_simparams &p) {
-  const double r0 = 0.6 / p.rei, rc = std::sqrt((double)p.rrCutEam);
-  return Spline{(float)r0, (float)(kSI / (rc - r0))};
+// First knot and interval width of a metal's splines.
+static void splineKnots(const sg_simparams &p, double &r0, double &h) {
+  r0 = 0.6 / p.rei;
+  h = (std::sqrt((double)p.rrCutEam) - r0) / kSI;
 }
 
 extern "C" int sg_diff_frame_params(const sg_simparams *in, sg_simparams *out) {
@@ -411,6 +793,104 @@ extern "C" int sg_diff_frame_params(const sg_simparams *in, sg_simparams *out) {
   return SG_OK;
 }
 
+// Blocks per SM that stream the reference forces of atoms without a pair: 2 keep the host link
+// busy and leave the SMs to the passes that run beside them.
+constexpr int kRefBlocks = 2;
+// From this many atoms the stream gets a launch of its own beside the passes; below, it is a few
+// blocks of the force pass, which saves the launch and two event waits.
+constexpr int kRefOwnLaunch = 65536;
+
+// The sums of an evaluation just read back.
+static double sumOf(const sg_diff *d, int q) {
+  double s = 0.0;
+  for (int c = 0; c < kSumCopies; c++) s += d->hostOut[c * kSumStride + q];
+  return s;
+}
+
+// Lays arrays out one after another (256-byte aligned) from base on; with base null only counts.
+struct Carver {
+  char *base;
+  size_t used = 0;
+  template <typename T> void take(T *&p, size_t n) {
+    if (base) p = reinterpret_cast<T *>(base + used);
+    used += (n * sizeof(T) + 255) & ~size_t(255);
+  }
+};
+
+// The packed rows, work lists and pairs of the positions and lists of d's context (built: it has
+// lists).
+static int packLists(sg_diff *d, bool built) {
+  sg_ctx *c = d->ctx;
+  DCK(cudaMemsetAsync(d->paired, 0, d->n, c->stream));
+  DCK(cudaMemsetAsync(d->counts, 0, 2 * sizeof(int), c->stream));
+  DCK(cudaMemsetAsync(d->totals, 0, 2 * sizeof(unsigned long long), c->stream));
+  DCK(cudaMemsetAsync(d->slotOf, 0xff, sizeof(int) * d->n, c->stream));
+  if (built) {
+    k_diff_slots<<<c->atomTab.n, 128, 0, c->stream>>>(c->atomTab.view(), c->rc, c->cellStart, c->sortIdx, d->slotOf);
+    // a row of carbon entries per warp in shared memory: one warp a block where rows are very long
+    const int warps = c->rowStride <= 3072 ? kDT / 32 : 1;
+    const size_t smem = sizeof(int) * warps * c->rowStride;
+    if (smem > 48 * 1024)
+      DCK(cudaFuncSetAttribute(k_diff_pack, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k_diff_pack<<<c->atomTab.n * (128 / warps), 32 * warps, smem, c->stream>>>(
+        c->atomTab.view(), c->rc, c->pos, c->nn, d->slotOf, c->nbl, c->rowStride, d->seg, d->paired);
+  }
+  k_diff_lists<<<c->atomTab.n, 128, 0, c->stream>>>(c->atomTab.view(), c->rc, c->cellStart, c->sortIdx, d->slotOf, built,
+                                                    d->paired, d->seg, d->metal, d->carbon, d->counts);
+  DCK(cudaGetLastError());
+  int counts[2];
+  DCK(cudaMemcpyAsync(counts, d->counts, sizeof counts, cudaMemcpyDeviceToHost, c->stream));
+  DCK(cudaStreamSynchronize(c->stream));
+  DiffWork *lists[2] = {d->metal, d->carbon};
+  DiffSlice *slices[2] = {d->metalSlices, d->carbonSlices};
+  for (int l = 0; l < 2; l++)
+    if (counts[l])
+      k_diff_slices<<<(counts[l] + kDT - 1) / kDT, kDT, 0, c->stream>>>(lists[l], counts[l], slices[l], d->totals);
+  DCK(cudaGetLastError());
+  unsigned long long pairs[2];
+  DCK(cudaMemcpyAsync(pairs, d->totals, sizeof pairs, cudaMemcpyDeviceToHost, c->stream));
+  DCK(cudaStreamSynchronize(c->stream));
+  d->nMetal = d->nCarbon = d->nOnce = 0;  // until the pairs are there
+  d->listed = true;
+  if (pairs[0] >= (1ull << 31)) return sg_fail(SG_ERR_NOMEM, "sg_diff: %llu pairs in one set of frames", pairs[0]);
+  if (pairs[0] > d->pairCap || pairs[1] > d->onceCap) {
+    // an eighth more than asked: a later set of positions rarely has as many more
+    const unsigned long long all = pairs[0] + pairs[0] / 8 + 1, once = pairs[1] + pairs[1] / 8 + 1;
+    auto lay = [&](Carver v) {
+      v.take(d->pairs.dir, all);
+      v.take(d->pairs.slot, all);
+      v.take(d->pairs.r, all);
+      v.take(d->pairs.w, all);
+      v.take(d->pairs.both, once);
+      v.take(d->pairs.rOnce, once);
+      v.take(d->pairs.place, once);
+      return v.used;
+    };
+    cudaFree(d->pairArena);
+    d->pairArena = nullptr;
+    d->pairCap = d->onceCap = 0;
+    if (cudaMalloc(&d->pairArena, lay(Carver{nullptr})) != cudaSuccess) {
+      cudaGetLastError();
+      d->pairArena = nullptr;
+      return sg_fail(SG_ERR_NOMEM, "sg_diff: memory for %llu pairs", all);
+    }
+    lay(Carver{static_cast<char *>(d->pairArena)});
+    d->pairCap = all;
+    d->onceCap = once;
+  }
+  d->nOnce = (int)pairs[1];
+  d->nMetal = counts[0];
+  d->nCarbon = counts[1];
+  for (int l = 0; l < 2; l++)
+    if (built && counts[l])
+      k_diff_pairs<<<(counts[l] + kDT / 32 - 1) / (kDT / 32), kDT, 0, c->stream>>>(
+          lists[l], slices[l], counts[l], c->rc, c->sortPos, c->nbl, c->rowStride, d->pairs);
+  if (built && d->nOnce)
+    k_diff_once<<<(counts[0] + kDT - 1) / kDT, kDT, 0, c->stream>>>(d->metal, d->metalSlices, counts[0], d->pairs);
+  DCK(cudaGetLastError());
+  return SG_OK;
+}
+
 extern "C" int sg_diff_create(const sg_simparams *frames, int n, int device, sg_diff **out) {
   if (!frames || n < 1 || !out) return sg_fail(SG_ERR_INVALID, "sg_diff_create: bad arguments");
   *out = nullptr;
@@ -427,33 +907,53 @@ extern "C" int sg_diff_create(const sg_simparams *frames, int n, int device, sg_
   o.device = device;
   sg_ctx *c = nullptr;
   if (int rc = sg_create(q.data(), n, &o, &c)) return rc;
-  sg_diff *d = new sg_diff;
+  size_t M = 0;
+  for (const RepConst &P : c->hrc) M += P.nMolMe;
+  sg_diff *d = new sg_diff(c->numSMs);
   d->ctx = c;
   d->nFrames = n;
   d->n = sg_num_atoms(c, -1);
-  d->sp = splineOf(q[0]);
-  d->p0 = q[0];
+  splineKnots(q[0], d->r0, d->h);
   const size_t N = d->n;
-  cudaError_t e = cudaSuccess;
-  if (e == cudaSuccess) e = cudaMalloc(&d->theta, sizeof(float) * kDP);
-  if (e == cudaSuccess) e = cudaMalloc(&d->Fp, sizeof(float) * N);
-  if (e == cudaSuccess) e = cudaMalloc(&d->force, sizeof(float4) * N);
-  if (e == cudaSuccess) e = cudaMalloc(&d->resid, sizeof(float4) * N);
-  if (e == cudaSuccess) e = cudaMalloc(&d->energy, sizeof(double) * n);
-  if (e == cudaSuccess) e = cudaMalloc(&d->grad, sizeof(double) * kDP);
-  if (e == cudaSuccess) e = cudaMalloc(&d->loss, sizeof(double));
+  d->outCap = kSums + std::max(n, c->numSMs * kRefBlocks);
+  auto lay = [&](Carver v) {
+    v.take(d->metal, M + 32);
+    v.take(d->carbon, N + 32);
+    v.take(d->metalSlices, M / 32 + 1);
+    v.take(d->carbonSlices, N / 32 + 1);
+    v.take(d->seg, N);
+    v.take(d->emb, N);
+    v.take(d->resid, N);
+    v.take(d->slotOf, N);
+    v.take(d->paired, N);
+    v.take(d->counts, 2);
+    v.take(d->totals, 2);
+    v.take(d->out, d->outCap);
+    v.take(d->model, 1);
+    return v.used;
+  };
+  auto layHost = [&](Carver v) {
+    v.take(d->hostModel, 1);
+    v.take(d->hostOut, d->outCap);
+    return v.used;
+  };
+  cudaError_t e = cudaMalloc(&d->arena, lay(Carver{nullptr}));
+  if (e == cudaSuccess) e = cudaMallocHost(&d->pinned, layHost(Carver{nullptr}));
   if (e != cudaSuccess) {
     sg_diff_destroy(d);
     return sg_fail(SG_ERR_NOMEM, "sg_diff_create: %s", cudaGetErrorString(e));
   }
+  lay(Carver{static_cast<char *>(d->arena)});
+  layHost(Carver{static_cast<char *>(d->pinned)});
   *out = d;
   return SG_OK;
 }
 
 extern "C" int sg_diff_destroy(sg_diff *d) {
   if (!d) return SG_OK;
-  cudaFree(d->theta); cudaFree(d->Fp); cudaFree(d->force); cudaFree(d->resid);
-  cudaFree(d->energy); cudaFree(d->grad); cudaFree(d->loss);
+  cudaFree(d->arena);
+  cudaFree(d->pairArena);
+  cudaFreeHost(d->pinned);
   if (d->ctx) sg_destroy(d->ctx);
   delete d;
   return SG_OK;
@@ -464,7 +964,10 @@ extern "C" int sg_diff_num_atoms(const sg_diff *d) { return d ? d->n : 0; }
 extern "C" int sg_diff_set_positions(sg_diff *d, const sg_float4 *r) {
   if (!d || !r) return sg_fail(SG_ERR_INVALID, "sg_diff_set_positions: null argument");
   if (int rc = sg_set_state(d->ctx, -1, r, nullptr, nullptr)) return rc;
-  return sg_build_lists(d->ctx);
+  const int built = sg_build_lists(d->ctx);  // a list that overflowed is used truncated
+  const std::string why = built ? sg_last_error() : "";
+  if (int rc = packLists(d, true)) return rc;
+  return built ? sg_fail(built, "%s", why.c_str()) : SG_OK;
 }
 
 extern "C" int sg_diff_init_theta(const sg_simparams *pp, double *theta) {
@@ -473,8 +976,8 @@ extern "C" int sg_diff_init_theta(const sg_simparams *pp, double *theta) {
   theta[0] = p.epsLJ;
   theta[1] = p.sigmaLJ;
   // least squares on 40 points per interval, normal equations solved by Cholesky in FP64
-  const Spline sp = splineOf(p);
-  const double r0 = sp.r0, h = 1.0 / sp.invH;
+  double r0, h;
+  splineKnots(p, r0, h);
   const int ns = 40 * kSI;
   std::vector<double> M(kSC * kSC, 0.0), rp(kSC, 0.0), rf(kSC, 0.0);
   for (int s = 0; s < ns; s++) {
@@ -515,82 +1018,138 @@ extern "C" int sg_diff_init_theta(const sg_simparams *pp, double *theta) {
   return SG_OK;
 }
 
-static int uploadTheta(sg_diff *d, const double *theta) {
-  float t[kDP];
-  for (int q = 0; q < kDP; q++) t[q] = (float)theta[q];
-  DCK(cudaMemcpyAsync(d->theta, t, sizeof t, cudaMemcpyHostToDevice, d->ctx->stream));
+// theta as the kernels read it, on its way to the device.  (Every call ends with its stream empty, so
+// the page-locked copy is free again.)
+static int uploadModel(sg_diff *d, const double *theta) {
+  if (!d->listed)  // no positions yet: every metal atom without a pair
+    if (int rc = packLists(d, false)) return rc;
+  DiffModel &m = *d->hostModel;
+  m.r0 = (float)d->r0;
+  m.invH = (float)(1.0 / d->h);
+  m.eps = (float)theta[0];
+  m.sig6 = (float)std::pow(theta[1], 6.0);
+  m.invSig = (float)(1.0 / theta[1]);
+  for (int k = 0; k < kSI; k++) {
+    const float knot = (float)(d->r0 + k * d->h);
+    const double t = (knot - d->r0) / d->h - k;  // the knot's own interval coordinate
+    m.knot[k] = make_float2(knot, (float)t);
+    for (int s = 0; s < 2; s++) {
+      // the B-spline sum of the interval as a cubic in t, moved to the rounded knot, per length
+      const double *c = theta + (s == 0 ? kPhi : kDen) + k;
+      const double a0 = (c[0] + 4.0 * c[1] + c[2]) / 6.0, a1 = (c[2] - c[0]) / 2.0, a2 = (c[0] - 2.0 * c[1] + c[2]) / 2.0,
+                   a3 = (c[3] - c[0] + 3.0 * (c[1] - c[2])) / 6.0;
+      (s == 0 ? m.phi : m.den)[k] = make_float4((float)(a0 + t * (a1 + t * (a2 + t * a3))), (float)((a1 + t * (2.0 * a2 + 3.0 * t * a3)) / d->h),
+                                 (float)((a2 + 3.0 * t * a3) / (d->h * d->h)), (float)(a3 / (d->h * d->h * d->h)));
+    }
+  }
+  DCK(cudaMemcpyAsync(d->model, &m, sizeof m, cudaMemcpyHostToDevice, d->ctx->stream));
   return SG_OK;
 }
 
-// Forward pass: F'(rho), forces of all atoms, frame energies, optionally dE/dtheta.
-static int forward(sg_diff *d, bool energyGrad) {
+// Slices of a work list of n atoms, a block each.
+static int slicesOf(int n) { return (n + 31) / 32; }
+
+// F'(rho) of the metal atoms, then the forces: packed into `force`, or (ref) the residuals and the
+// loss, with refBlocks blocks for the atoms without a pair (their sums at out + kSums) in the same
+// launch or (own) in one on the side stream.  That one starts when the reference forces of the atoms
+// with pairs are there: a fetch beside it would share the host link and hold up the force pass by
+// most of the transfer (64 frames of 20,432 atoms: 281 us an evaluation instead of 236).
+static int forces(sg_diff *d, float *force, const float *ref, float scale, int refBlocks, bool own) {
   sg_ctx *c = d->ctx;
-  DCK(cudaMemsetAsync(d->energy, 0, sizeof(double) * d->nFrames, c->stream));
-  DCK(cudaMemsetAsync(d->grad, 0, sizeof(double) * kDP, c->stream));
-  DCK(cudaMemsetAsync(d->force, 0, sizeof(float4) * d->n, c->stream));
-  if (c->metalTabT.n) {
-    k_diff_rho<<<c->metalTabT.n, 128, 0, c->stream>>>(c->metalTabT.view(), c->rc, c->pos, c->nn, c->nbl,
-                                                      c->rowStride, d->theta, d->sp, d->Fp, d->energy);
-    k_diff_force_metal<<<c->metalTabT.n, 128, 0, c->stream>>>(c->metalTabT.view(), c->rc, c->pos, c->nn, c->nbl,
-                                                              c->rowStride, d->theta, d->sp, d->Fp, d->force,
-                                                              d->energy, energyGrad ? d->grad : nullptr);
+  const int nm = slicesOf(d->nMetal);
+  // k_diff_rho also clears the sums, so it runs (one block) without metal too
+  const int refGather = ref ? std::min((d->n + kPassThreads - 1) / kPassThreads, c->numSMs * kRefBlocks) : 0;
+  DCK(launchK(false, k_diff_rho<false>, std::max(1, std::min(nm, d->most.rho) + refGather), kPassThreads, 0, c->stream,
+              d->model, d->metal, d->metalSlices, d->nMetal, c->rc, d->pairs.r, d->emb, nullptr, d->out, ref, d->n,
+              d->paired, d->slotOf, d->resid, refGather));
+  if (own) {
+    DCK(cudaEventRecord(c->evFork, c->stream));
+    DCK(cudaStreamWaitEvent(c->side, c->evFork, 0));
+    k_diff_ref<<<refBlocks, kDT, 0, c->side>>>(ref, d->n, d->paired, d->out + kSums);
+    DCK(cudaGetLastError());
+    DCK(cudaEventRecord(c->evJoin, c->side));
+    refBlocks = 0;
   }
-  if (c->carbonTab.n)
-    k_diff_force_carbon<<<c->carbonTab.n, 128, 0, c->stream>>>(c->carbonTab.view(), c->rc, c->pos, c->nn,
-                                                               c->nbl, c->rowStride, d->theta, d->force);
-  DCK(cudaGetLastError());
+  const int blocks = std::min(nm + slicesOf(d->nCarbon), ref ? d->most.residual : d->most.force) + refBlocks;
+  if (blocks > 0)
+    DCK(launchK(true, ref ? k_diff_force<true> : k_diff_force<false>, blocks, kPassThreads, 0, c->stream, d->model, d->metal,
+                d->metalSlices, d->nMetal, d->carbon, d->carbonSlices, d->nCarbon, c->sortIdx, d->pairs, d->emb, force, ref,
+                scale, d->resid, d->out, d->out + kSums, d->n, d->paired, refBlocks));
+  return SG_OK;
+}
+
+// The parameter sums of an energy or loss evaluation, after its densities (and residuals).
+template <bool LOSS>
+static int parameterSums(sg_diff *d) {
+  sg_ctx *c = d->ctx;
+  if (d->nMetal)
+    DCK(launchK(true, k_diff_along<LOSS>, std::min(slicesOf(d->nMetal), LOSS ? d->most.along : d->most.lj), kPassThreads, 0,
+                c->stream, d->model, d->metal, d->metalSlices, d->nMetal, d->pairs, d->resid, d->emb, d->out));
+  if (d->nOnce)
+    DCK(launchK(true, k_diff_sums<LOSS>, std::min((d->nOnce + kDT - 1) / kDT, LOSS ? d->most.lossSums : d->most.energySums),
+                kDT, 0, c->stream, d->model, d->pairs, d->nOnce, d->emb, d->out));
   return SG_OK;
 }
 
 extern "C" int sg_diff_energy(sg_diff *d, const double *theta, double *energy, double *grad) {
   if (!d || !theta) return sg_fail(SG_ERR_INVALID, "sg_diff_energy: null argument");
-  int rc;
-  if ((rc = uploadTheta(d, theta)) || (rc = forward(d, grad != nullptr))) return rc;
-  if (energy)
-    DCK(cudaMemcpyAsync(energy, d->energy, sizeof(double) * d->nFrames, cudaMemcpyDeviceToHost, d->ctx->stream));
-  if (grad) DCK(cudaMemcpyAsync(grad, d->grad, sizeof(double) * kDP, cudaMemcpyDeviceToHost, d->ctx->stream));
-  DCK(cudaStreamSynchronize(d->ctx->stream));
+  sg_ctx *c = d->ctx;
+  if (int rc = uploadModel(d, theta)) return rc;
+  const size_t bytes = sizeof(double) * (kSums + d->nFrames);
+  DCK(cudaMemsetAsync(d->out, 0, bytes, c->stream));
+  if (d->nMetal) {
+    DCK(launchK(false, k_diff_rho<true>, std::min(slicesOf(d->nMetal), d->most.energy), kPassThreads, 0, c->stream, d->model, d->metal, d->metalSlices, d->nMetal, c->rc,
+                d->pairs.r, d->emb, d->out + kSums, d->out, nullptr, d->n, d->paired, d->slotOf, d->resid, 0));
+    if (grad)
+      if (int rc = parameterSums<false>(d)) return rc;
+  }
+  DCK(cudaMemcpyAsync(d->hostOut, d->out, bytes, cudaMemcpyDeviceToHost, c->stream));
+  DCK(cudaStreamSynchronize(c->stream));
+  if (energy) memcpy(energy, d->hostOut + kSums, sizeof(double) * d->nFrames);
+  if (grad)
+    for (int q = 0; q < kDP; q++) grad[q] = sumOf(d, q);
   return SG_OK;
 }
 
-extern "C" int sg_diff_forces(sg_diff *d, const double *theta, float *forces) {
-  if (!d || !theta || !forces) return sg_fail(SG_ERR_INVALID, "sg_diff_forces: null argument");
-  int rc;
-  if ((rc = uploadTheta(d, theta)) || (rc = forward(d, false))) return rc;
+extern "C" int sg_diff_forces(sg_diff *d, const double *theta, float *out) {
+  if (!d || !theta || !out) return sg_fail(SG_ERR_INVALID, "sg_diff_forces: null argument");
   sg_ctx *c = d->ctx;
-  k_pack3<<<(d->n + 255) / 256, 256, 0, c->stream>>>(d->force, c->stage, d->n);
-  DCK(cudaGetLastError());
-  DCK(cudaMemcpyAsync(forces, c->stage, sizeof(float) * 3 * d->n, cudaMemcpyDeviceToHost, c->stream));
+  DCK(cudaMemsetAsync(c->stage, 0, sizeof(float) * 3 * d->n, c->stream));  // atoms without a pair
+  if (int rc = uploadModel(d, theta)) return rc;
+  if (int rc = forces(d, c->stage, nullptr, 0.f, 0, false)) return rc;
+  DCK(cudaMemcpyAsync(out, c->stage, sizeof(float) * 3 * d->n, cudaMemcpyDeviceToHost, c->stream));
   DCK(cudaStreamSynchronize(c->stream));
   return SG_OK;
 }
 
+// The reference forces are read in place where the device reads host memory directly (their
+// transfer then overlaps the passes: only the paired atoms' are needed early), else copied first.
 extern "C" int sg_diff_force_matching(sg_diff *d, const double *theta, const float *ref, double *loss,
                                       double *grad) {
   if (!d || !theta || !ref) return sg_fail(SG_ERR_INVALID, "sg_diff_force_matching: null argument");
   sg_ctx *c = d->ctx;
-  int rc;
-  if ((rc = uploadTheta(d, theta))) return rc;
-  DCK(cudaMemcpyAsync(c->stage, ref, sizeof(float) * 3 * d->n, cudaMemcpyHostToDevice, c->stream));
-  k_unpack3<<<(d->n + 255) / 256, 256, 0, c->stream>>>(c->stage, d->resid, d->n);
-  DCK(cudaGetLastError());
-  if ((rc = forward(d, false))) return rc;
-  DCK(cudaMemsetAsync(d->loss, 0, sizeof(double), c->stream));
+  if (int rc = uploadModel(d, theta)) return rc;
   const double inv3N = 1.0 / (3.0 * d->n);
-  k_diff_resid<<<(d->n + 255) / 256, 256, 0, c->stream>>>(d->n, d->force, d->resid, (float)(2.0 * inv3N), inv3N,
-                                                          d->loss);
-  DCK(cudaGetLastError());
-  if (grad) {
-    DCK(cudaMemsetAsync(d->grad, 0, sizeof(double) * kDP, c->stream));
-    if (c->metalTabT.n)
-      k_diff_adjoint<<<c->metalTabT.n, 128, 0, c->stream>>>(c->metalTabT.view(), c->rc, c->pos, c->nn, c->nbl,
-                                                            c->rowStride, d->theta, d->sp, d->resid, d->grad);
-    DCK(cudaGetLastError());
-    DCK(cudaMemcpyAsync(grad, d->grad, sizeof(double) * kDP, cudaMemcpyDeviceToHost, c->stream));
+  const float *src = ref;
+  if (!c->hostDirect) {
+    DCK(cudaMemcpyAsync(c->stage, ref, sizeof(float) * 3 * d->n, cudaMemcpyHostToDevice, c->stream));
+    src = c->stage;
   }
-  if (loss) DCK(cudaMemcpyAsync(loss, d->loss, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  const bool own = d->n >= kRefOwnLaunch;
+  const int refBlocks = std::max(1, std::min((d->n * 3 / 4 + kDT - 1) / kDT, c->numSMs * kRefBlocks));
+  int rc = forces(d, nullptr, src, (float)(2.0 * inv3N), refBlocks, own);
+  if (!rc && grad) rc = parameterSums<true>(d);
+  // joined whatever happened: the stream reads the caller's array until k_diff_ref is done
+  if (own) DCK(cudaStreamWaitEvent(c->stream, c->evJoin, 0));
+  if (!rc) DCK(cudaMemcpyAsync(d->hostOut, d->out, sizeof(double) * (kSums + refBlocks), cudaMemcpyDeviceToHost, c->stream));
   DCK(cudaStreamSynchronize(c->stream));
+  if (rc) return rc;
+  if (loss) {
+    double s = sumOf(d, kDP);
+    for (int b = 0; b < refBlocks; b++) s += d->hostOut[kSums + b];
+    *loss = s * inv3N;
+  }
   if (grad)
-    for (int q = 0; q < kDP; q++) grad[q] = -grad[q];  // dL/dtheta = -dD/dtheta
+    for (int q = 0; q < kDP; q++) grad[q] = -sumOf(d, q);  // dL/dtheta = -dD/dtheta
   return SG_OK;
 }
