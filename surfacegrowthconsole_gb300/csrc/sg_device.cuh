@@ -41,8 +41,6 @@ constexpr int kRelMax = 48;       // relevant-list capacity per carbon atom
 constexpr int kShortMax = 8;      // close-list capacity per carbon atom (a multiple of 4)
 constexpr int kRelPosLimit = 256; // relevant-list entries record list positions below this
 constexpr int kMaxReplicaAtoms = 1 << 24;  // atoms of one replica (relevant entries index 24 bits)
-constexpr int kHeavyCell = 16;    // list build: default home atoms per work item (larger cells split)
-constexpr int kHeavyChunk = 8;    // sizes the item list of the fixed-size scratch (>= kHeavyCell / 2)
 constexpr int kScanCells = 128;   // cells per block of the single-pass cell scan and ordering (or 2x)
 constexpr int kScanRankThreads = 512;  // threads of that block (the ordering uses all of them)
 constexpr int kMixThreads = 512;  // MIXED step reduction: threads per block

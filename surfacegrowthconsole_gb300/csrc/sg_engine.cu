@@ -355,7 +355,7 @@ extern "C" int sg_create(const sg_simparams *params, int n_replicas, const sg_op
   AL(c->st, n_replicas);
   AL(c->pos, N); AL(c->vel, N); AL(c->acc, N); AL(c->sortPos, N);
   if (c->opt.mode == SG_MODE_MIXED) AL(c->posLo, N);
-  AL(c->cellOf, N); AL(c->slot, N); AL(c->tmpIdx, N); AL(c->sortIdx, N);
+  AL(c->cellOf, N); AL(c->slot, N); AL(c->sortIdx, N);
   AL(c->cellCount, (size_t)c->ctot); AL(c->cellStart, (size_t)c->ctot);
   AL(c->nn, N); AL(c->ns, N);
   AL(c->sl, N * kShortMax);
@@ -466,8 +466,7 @@ extern "C" int sg_create(const sg_simparams *params, int n_replicas, const sg_op
       sg_destroy(c);
       return rc;
     }
-    if ((rc = devAllocT(c, &c->tileSum, std::max<size_t>(tr.size(), 1))) ||
-        (rc = devAllocT(c, &c->dTileFirst, n_replicas)) ||
+    if ((rc = devAllocT(c, &c->dTileFirst, n_replicas)) ||
         (rc = devAllocT(c, &c->blockCount, std::max<size_t>(tr.size() * (kCellTile / kScanCells), 1)))) {
       sg_destroy(c);
       return rc;

@@ -45,7 +45,7 @@ struct sg_ctx {
   RepState *st = nullptr;
   float4 *pos = nullptr, *vel = nullptr, *acc = nullptr, *posLo = nullptr, *sortPos = nullptr;
   int *cellOf = nullptr, *slot = nullptr, *cellCount = nullptr, *cellStart = nullptr;
-  int *tmpIdx = nullptr, *sortIdx = nullptr, *nn = nullptr, *nbl = nullptr, *ns = nullptr, *sl = nullptr;
+  int *sortIdx = nullptr, *nn = nullptr, *nbl = nullptr, *ns = nullptr, *sl = nullptr;
   int *nrl = nullptr;
   unsigned *rl = nullptr;  // relevant lists (relPack entries)
   int nebrGrid = 0;
@@ -58,7 +58,7 @@ struct sg_ctx {
   int2 *heavyItems = nullptr;
   float *rho = nullptr, *dF = nullptr, *Fv = nullptr, *fric = nullptr;
   float *partial = nullptr, *partialCmv = nullptr;
-  int *dRedFirst = nullptr, *dCmvFirst = nullptr, *tileSum = nullptr, *dTileFirst = nullptr;
+  int *dRedFirst = nullptr, *dCmvFirst = nullptr, *dTileFirst = nullptr;
   unsigned *hist = nullptr;
   unsigned long long *histExt = nullptr;
   int4 *rdfPairs = nullptr;  // RDF extension: {replica, first A atom, first B atom} per tile pair

@@ -9,8 +9,6 @@ namespace sg {
 __global__ void k_integrate_first(BlockTab tab, const RepConst *rc, RepState *st, float4 *pos,
                                   float4 *vel, const float4 *acc, int *cellOf, int *slot,
                                   int *cellCount, int forceRebuild, int *bucket, int cap, int *blockCount);
-__global__ void k_cell_count(BlockTab tab, const RepConst *rc, const float4 *pos, int *cellOf,
-                             int *slot, int *cellCount);
 __global__ void k_cell_bucket(BlockTab tab, const RepConst *rc, const float4 *pos, int *cellOf, int *slot,
                               int *cellCount, int *bucket, int cap, int *blockCount, int2 *spill, int *spillCount);
 __global__ void k_build_nebr_atoms(BlockTab tab, const RepConst *rc, RepState *st, const int *cellOf,
@@ -23,19 +21,6 @@ cudaError_t launchScanRank(bool pdl, int cells, int grid, cudaStream_t s, const 
                            int cap, int forceRebuild, int *active, int2 *heavy, int *work, int itemAtoms,
                            const int *blockCount, const int *bucket, const int2 *spill, const int *cellOf,
                            const float4 *pos, int *sortIdx, float4 *sortPos, int *nn, int *ns, int *nrl);
-__global__ void k_scan_tiles(BlockTab tab, const RepConst *rc, const RepState *st,
-                             const int *cellCount, int *tileSum, int forceRebuild);
-__global__ void k_scan_tile_prefix(const RepConst *rc, const RepState *st, const int *tileFirst,
-                                   int *tileSum, int forceRebuild, int *work);
-__global__ void k_scan_final(BlockTab tab, const RepConst *rc, RepState *st, int *cellCount,
-                             const int *tileSum, int *cellStart, int blockSizeCap, int forceRebuild,
-                             int *active, int2 *heavy, int *work, int itemAtoms);
-__global__ void k_scatter(BlockTab tab, const RepConst *rc, RepState *st, const int *cellOf,
-                          const int *slot, const int *cellStart, int *tmpIdx, int *nn, int *ns, int *nrl,
-                          int forceRebuild);
-__global__ void k_rank(BlockTab tab, const RepConst *rc, const RepState *st, const int *cellOf,
-                       const int *cellStart, const int *tmpIdx, const float4 *pos, int *sortIdx,
-                       float4 *sortPos, int forceRebuild);
 // work[0]: next work item to take, work[1]: length of the cell list `active`, work[2]: length
 // of the home-chunk list `heavy` (all reset before the scan of every rebuild).
 __global__ void k_build_nebr(const int *tileRep, const int *active, const int2 *heavy, int *work, const RepConst *rc, RepState *st,
@@ -53,6 +38,9 @@ __global__ void k_rho(BlockTab tab, const RepConst *rc, const float4 *pos, const
 __global__ void k_force_metal(BlockTab tab, const RepConst *rc, float4 *pos, float4 *acc,
                               const int *nn, const int *nbl, const float *dF, const float *Fv,
                               float *fric, int rowStride);
+__global__ void k_force_both(BlockTab metal, BlockTab carbon, const RepConst *rc, float4 *pos, float4 *acc, const int *nn,
+                             const int *nbl, const int *ns, const int *sl, const int *nrl, const unsigned *rl,
+                             const float *dF, const float *Fv, float *fric, int rowStride);
 // the metal chain (k_rho, k_force_metal) with mt lanes per atom (4, 8, 16, 32) on the table of
 // 128 / mt atoms per block
 void launchMetalChain(bool pdl, int mt, int grid, int stagedGrid, size_t stagedSmem, cudaStream_t s, BlockTab tab, const RepConst *rc, float4 *pos,

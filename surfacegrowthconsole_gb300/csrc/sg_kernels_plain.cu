@@ -105,20 +105,6 @@ __global__ void k_integrate_first(BlockTab tab, const RepConst *__restrict__ rc,
   if (forceRebuild || S->nebrNow) binAtom(P, g, r, cellOf, slot, cellCount, bucket, cap, blockCount);
 }
 
-// Histogram pass alone (used when lists are rebuilt outside a step).
-__global__ void k_cell_count(BlockTab tab, const RepConst *__restrict__ rc,
-                             const float4 *__restrict__ pos, int *__restrict__ cellOf,
-                             int *__restrict__ slot, int *__restrict__ cellCount) {
-  const int rep = tab.rep[blockIdx.x];
-  const RepConst &P = rc[rep];
-  const int g = tab.start[blockIdx.x] + threadIdx.x;
-  if (g >= P.atomOff + P.nMol) return;
-  const float4 r = pos[g];
-  const int c = cellIndex(P, r.x, r.y, r.z);
-  cellOf[g] = c;
-  if (c >= 0) slot[g] = atomicAdd(&cellCount[P.cellOff + c], 1);
-}
-
 // Histogram and bucket pass alone (lists rebuilt outside a step).
 __global__ void k_cell_bucket(BlockTab tab, const RepConst *__restrict__ rc, const float4 *__restrict__ pos,
                               int *__restrict__ cellOf, int *__restrict__ slot, int *__restrict__ cellCount,
@@ -132,226 +118,6 @@ __global__ void k_cell_bucket(BlockTab tab, const RepConst *__restrict__ rc, con
   binAtom(P, g, pos[g], cellOf, slot, cellCount, bucket, cap, blockCount, spill, spillCount);
 }
 
-
-// ============================================================================================
-// Counting sort of atoms by cell: exclusive scan of the per-cell counts, in three passes
-// (tile sums, per-replica tile prefix, in-tile scan), then scatter and in-cell ordering.
-// ============================================================================================
-__global__ void k_scan_tiles(BlockTab tab, const RepConst *__restrict__ rc, const RepState *st,
-                             const int *__restrict__ cellCount, int *__restrict__ tileSum,
-                             int forceRebuild) {
-  pdlEnter();
-  const int rep = tab.rep[blockIdx.x];
-  if (!rebuilding(st + rep, forceRebuild)) return;
-  const RepConst &P = rc[rep];
-  const int c0 = tab.start[blockIdx.x];  // local cell index of the tile start
-  int s = 0;
-  for (int c = c0 + threadIdx.x; c < c0 + kCellTile; c += blockDim.x) s += cellCount[P.cellOff + c];
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  __shared__ int ws[32];
-  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    int v = (threadIdx.x < (blockDim.x >> 5)) ? ws[threadIdx.x] : 0;
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (threadIdx.x == 0) tileSum[blockIdx.x] = v;
-  }
-}
-
-// One block per replica: exclusive prefix over the replica's tiles (tiles of a replica are
-// consecutive blocks of the tile table starting at tileFirst[rep]).  Block 0 also clears the
-// list build's work counters (work, if not NULL) for k_scan_final and k_build_nebr.
-__global__ void k_scan_tile_prefix(const RepConst *__restrict__ rc, const RepState *st,
-                                   const int *__restrict__ tileFirst, int *__restrict__ tileSum,
-                                   int forceRebuild, int *__restrict__ work) {
-  pdlEnter();
-  if (work && blockIdx.x == 0 && threadIdx.x < 3) work[threadIdx.x] = 0;
-  const int rep = blockIdx.x;
-  if (!rebuilding(st + rep, forceRebuild)) return;
-  const RepConst &P = rc[rep];
-  const int t0 = tileFirst[rep];
-  const int nt = P.ncellsPad / kCellTile;
-  __shared__ int carry;
-  __shared__ int ws[32];
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  for (int base = 0; base < nt; base += blockDim.x) {
-    const int t = base + threadIdx.x;
-    int v = (t < nt) ? tileSum[t0 + t] : 0;
-    // inclusive warp scan
-    int x = v;
-    for (int o = 1; o < 32; o <<= 1) {
-      int y = __shfl_up_sync(0xffffffffu, x, o);
-      if ((threadIdx.x & 31) >= o) x += y;
-    }
-    if ((threadIdx.x & 31) == 31) ws[threadIdx.x >> 5] = x;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-      int w = (threadIdx.x < (blockDim.x >> 5)) ? ws[threadIdx.x] : 0;
-      for (int o = 1; o < 32; o <<= 1) {
-        int y = __shfl_up_sync(0xffffffffu, w, o);
-        if (threadIdx.x >= o) w += y;
-      }
-      ws[threadIdx.x] = w;
-    }
-    __syncthreads();
-    const int warpPrefix = (threadIdx.x >= 32) ? ws[(threadIdx.x >> 5) - 1] : 0;
-    const int excl = carry + warpPrefix + x - v;
-    if (t < nt) tileSum[t0 + t] = excl;
-    __syncthreads();
-    if (threadIdx.x == blockDim.x - 1) carry = excl + v;
-    __syncthreads();
-  }
-}
-
-// In-tile exclusive scan; writes global cellStart (index into the sorted arrays) and clears
-// the counts for the next rebuild.  Also records the largest cell occupancy.
-__global__ void k_scan_final(BlockTab tab, const RepConst *__restrict__ rc, RepState *st,
-                             int *__restrict__ cellCount, const int *__restrict__ tileSum,
-                             int *__restrict__ cellStart, int blockSizeCap, int forceRebuild,
-                             int *__restrict__ active, int2 *__restrict__ heavy, int *__restrict__ work,
-                             int itemAtoms) {
-  pdlEnter();
-  const int rep = tab.rep[blockIdx.x];
-  RepState *S = st + rep;
-  if (!rebuilding(S, forceRebuild)) return;
-  const RepConst &P = rc[rep];
-  const int c0 = tab.start[blockIdx.x];
-  constexpr int kPer = kCellTile / 256;  // launched with 256 threads
-  int v[kPer];
-  int sum = 0, occ = 0, over = 0;
-  const int cb = P.cellOff + c0 + threadIdx.x * kPer;
-#pragma unroll
-  for (int i = 0; i < kPer; i++) {
-    v[i] = cellCount[cb + i];
-    occ = max(occ, v[i]);
-    over += (v[i] > blockSizeCap) ? 1 : 0;
-    sum += v[i];
-  }
-  __shared__ int ws[8];
-  int x = sum;
-  for (int o = 1; o < 32; o <<= 1) {
-    int y = __shfl_up_sync(0xffffffffu, x, o);
-    if ((threadIdx.x & 31) >= o) x += y;
-  }
-  if ((threadIdx.x & 31) == 31) ws[threadIdx.x >> 5] = x;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    int w = (threadIdx.x < 8) ? ws[threadIdx.x] : 0;
-    for (int o = 1; o < 8; o <<= 1) {
-      int y = __shfl_up_sync(0xffffffffu, w, o);
-      if (threadIdx.x >= o) w += y;
-    }
-    if (threadIdx.x < 8) ws[threadIdx.x] = w;
-  }
-  __syncthreads();
-  int run = P.atomOff + tileSum[blockIdx.x] + ((threadIdx.x >= 32) ? ws[(threadIdx.x >> 5) - 1] : 0) + x - sum;
-#pragma unroll
-  for (int i = 0; i < kPer; i++) {
-    cellStart[cb + i] = run;
-    run += v[i];
-    cellCount[cb + i] = 0;
-  }
-  // work items of the list build (any order): a cell of up to itemAtoms atoms is one item; a
-  // cell of n > itemAtoms atoms is split into k = ceil(n / itemAtoms) items of n / k home atoms
-  // (rounded), queued apart so that the list build takes them first.  A split item is
-  // {cell, first home atom << 16 | home atoms}.
-  int nLight = 0, nHeavy = 0;
-#pragma unroll
-  for (int i = 0; i < kPer; i++) {
-    if (v[i] > 0 && c0 + threadIdx.x * kPer + i < P.ncells) {
-      if (v[i] > itemAtoms) nHeavy += (v[i] + itemAtoms - 1) / itemAtoms;
-      else nLight++;
-    }
-  }
-  int preL = nLight, preH = nHeavy;
-  for (int o = 1; o < 32; o <<= 1) {
-    const int yl = __shfl_up_sync(0xffffffffu, preL, o);
-    const int yh = __shfl_up_sync(0xffffffffu, preH, o);
-    if ((threadIdx.x & 31) >= o) { preL += yl; preH += yh; }
-  }
-  const int sumL = __shfl_sync(0xffffffffu, preL, 31), sumH = __shfl_sync(0xffffffffu, preH, 31);
-  int baseL = 0, baseH = 0;
-  if ((threadIdx.x & 31) == 31) {
-    if (sumL > 0) baseL = atomicAdd(&work[1], sumL);
-    if (sumH > 0) baseH = atomicAdd(&work[2], sumH);
-  }
-  int outL = __shfl_sync(0xffffffffu, baseL, 31) + preL - nLight;
-  int outH = __shfl_sync(0xffffffffu, baseH, 31) + preH - nHeavy;
-#pragma unroll
-  for (int i = 0; i < kPer; i++) {
-    if (v[i] > 0 && c0 + threadIdx.x * kPer + i < P.ncells) {
-      if (v[i] > itemAtoms) {
-        const int k = (v[i] + itemAtoms - 1) / itemAtoms;
-        for (int j = 0; j < k; j++) {
-          const int h0 = j * v[i] / k, h1 = (j + 1) * v[i] / k;
-          heavy[outH++] = make_int2(cb + i, (h0 << 16) | (h1 - h0));
-        }
-      } else {
-        active[outL++] = cb + i;
-      }
-    }
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    occ = max(occ, __shfl_xor_sync(0xffffffffu, occ, o));
-    over += __shfl_xor_sync(0xffffffffu, over, o);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    if (occ > 0) atomicMax(&S->maxCellOcc, occ);
-    if (over > 0) {
-      atomicAdd(&S->cellOverflow, over);
-      setFlag(S, 11 /*SG_ERR_CELL_OVERFLOW*/);
-    }
-  }
-}
-
-// Scatter atoms into their cell segments in arrival order.
-__global__ void k_scatter(BlockTab tab, const RepConst *__restrict__ rc, RepState *st,
-                          const int *__restrict__ cellOf, const int *__restrict__ slot,
-                          const int *__restrict__ cellStart, int *__restrict__ tmpIdx,
-                          int *__restrict__ nn, int *__restrict__ ns, int *__restrict__ nrl,
-                          int forceRebuild) {
-  pdlEnter();
-  const int rep = tab.rep[blockIdx.x];
-  RepState *S = st + rep;
-  if (!rebuilding(S, forceRebuild)) return;
-  const RepConst &P = rc[rep];
-  const int g = tab.start[blockIdx.x] + threadIdx.x;
-  if (g >= P.atomOff + P.nMol) return;
-  const int c = cellOf[g];
-  if (c >= 0) {
-    tmpIdx[cellStart[P.cellOff + c] + slot[g]] = g;
-  } else {
-    nn[g] = 0;  // an atom outside the grid has no neighbours (the reference clears NN)
-    ns[g] = 0;
-    nrl[g] = 0;
-    atomicAdd(&S->cellRange, 1);
-  }
-}
-
-// Order each cell by ascending atom index: the rank of an atom is the number of atoms of its
-// cell with a smaller index.  Writes the sorted index and a sorted position copy whose w holds
-// the atom index (as int bits) for the neighbour search.
-__global__ void k_rank(BlockTab tab, const RepConst *__restrict__ rc, const RepState *st,
-                       const int *__restrict__ cellOf, const int *__restrict__ cellStart,
-                       const int *__restrict__ tmpIdx, const float4 *__restrict__ pos,
-                       int *__restrict__ sortIdx, float4 *__restrict__ sortPos, int forceRebuild) {
-  pdlEnter();
-  const int rep = tab.rep[blockIdx.x];
-  if (!rebuilding(st + rep, forceRebuild)) return;
-  const RepConst &P = rc[rep];
-  const int g = tab.start[blockIdx.x] + threadIdx.x;
-  if (g >= P.atomOff + P.nMol) return;
-  const int c = cellOf[g];
-  if (c < 0) return;
-  const int b = cellStart[P.cellOff + c], e = cellStart[P.cellOff + c + 1];
-  int rank = 0;
-  for (int q = b; q < e; q++) rank += (tmpIdx[q] < g) ? 1 : 0;
-  sortIdx[b + rank] = g;
-  float4 r = pos[g];
-  r.w = __int_as_float(g);
-  sortPos[b + rank] = r;
-}
 
 // k_scan_rank: one block of kScanRankThreads threads per CELLS cells (sg_lists.cuh).
 template <int CELLS>
@@ -418,6 +184,27 @@ __global__ void __launch_bounds__(kNebrWarps * 32) k_build_nebr_lanes(SG_NEBR_PA
 }  // namespace sg
 #define SG_KN(name) name
 #include "sg_forces.cuh"
+
+namespace sg {
+
+// Metal forces (the first metal.nblocks blocks) and carbon forces in one launch, for a caller with
+// one stream: neither needs the other, and a system of up to 16,384 atoms leaves the GPU room for
+// both at once.
+__global__ void __launch_bounds__(128, 8) k_force_both(BlockTab metal, BlockTab carbon, const RepConst *__restrict__ rc,
+                                                       float4 *__restrict__ pos, float4 *__restrict__ acc,
+                                                       const int *__restrict__ nn, const int *__restrict__ nbl,
+                                                       const int *__restrict__ ns, const int *__restrict__ sl,
+                                                       const int *__restrict__ nrl, const unsigned *__restrict__ rl,
+                                                       const float *__restrict__ dF, const float *__restrict__ Fv,
+                                                       float *__restrict__ fric, int rowStride) {
+  pdlEnter();
+  if ((int)blockIdx.x < metal.nblocks)
+    forceMetalBody<kMT>(blockIdx.x, rc[metal.rep[blockIdx.x]], metal, pos, acc, nn, nbl, dF, Fv, fric, rowStride);
+  else
+    carbonBody(blockIdx.x - metal.nblocks, carbon, rc, pos, acc, nn, nbl, ns, sl, nrl, rl, rowStride);
+}
+
+}  // namespace sg
 namespace sg {
 
 // ============================================================================================

@@ -10,10 +10,11 @@
 // SG_NOALLOC_SCRATCH_BYTES, which every GPU that loads the library holds until the process
 // exits.
 //
-// The work is the same kernel chain as sg_build_lists + sg_compute_forces of a context: cell
-// counting sort, neighbour list, EAM density, metal and carbon forces.
+// The work is that of sg_build_lists + sg_compute_forces of a context: atoms sorted by cell,
+// neighbour list, EAM density, metal and carbon forces, in five launches.
 #include <cuda_runtime.h>
 
+#include <cstddef>
 #include <cstring>
 #include <mutex>
 
@@ -28,10 +29,16 @@ namespace {
 
 constexpr size_t kScratchBytes = SG_NOALLOC_SCRATCH_BYTES;
 constexpr int kBs = 128;
-constexpr int kMaxBlocks = (SG_NOALLOC_MAX_ATOMS + kBs - 1) / kBs;
 // table capacity: the metal pass has the smallest blocks (kMetalPerBlock atoms)
 constexpr int kMaxTabBlocks = (SG_NOALLOC_MAX_ATOMS + kMetalPerBlock - 1) / kMetalPerBlock;
 constexpr int kMaxTiles = SG_NOALLOC_MAX_CELLS / kCellTile;
+// home atoms per work item of the list build: 4, so that a small system's warps have little to do in
+// sequence (a call on 2,217 / 15,883 atoms: 54.8 / 67.2 us; 8 as in the step, 56.7 / 67.7)
+constexpr int kItem = kMinItemAtoms;
+constexpr int kSortCells = 512;         // cells per block of the sort
+constexpr int kSortThreads = 1024;
+constexpr int kBuildBlocks = 7 * 152;  // the list build's: its blocks resident at once on a GB300
+static_assert(SG_NOALLOC_MAX_ATOMS < (1 << 15) && kSortCells <= (1 << 16), "the sort packs cell and atom in a word");
 
 // The scratch of every call on this device.  Host code must not take its address directly:
 // the host-side name is only a stand-in; the device address comes from cudaGetSymbolAddress.
@@ -39,8 +46,8 @@ static __device__ __align__(256) unsigned char g_scratch[kScratchBytes];
 
 // Carving of the scratch array (offsets in bytes, each 256-byte aligned).
 struct Carve {
-  size_t rc, st, tabRep, tabStart, tileRep, tileStart, tileFirst, tileSum, cellCount, cellStart;
-  size_t cellOf, slot, tmpIdx, sortIdx, nn, ns, sl, sortPos, rho, dF, Fv, fric, nbl, nrl, rl, active, heavy, work, total;
+  size_t rc, st, tabRep, tabStart, tileRep, cellStart;
+  size_t cellOf, sortIdx, nn, ns, sl, sortPos, rho, dF, Fv, fric, nbl, nrl, rl, active, heavy, work, total;
 };
 constexpr size_t up(size_t x) { return (x + 255) & ~size_t(255); }
 constexpr Carve carve() {
@@ -52,14 +59,8 @@ constexpr Carve carve() {
   c.tabRep = o; o += up(3 * kMaxTabBlocks * sizeof(int));    // atom, metal, carbon tables
   c.tabStart = o; o += up(3 * kMaxTabBlocks * sizeof(int));
   c.tileRep = o; o += up(kMaxTiles * sizeof(int));
-  c.tileStart = o; o += up(kMaxTiles * sizeof(int));
-  c.tileFirst = o; o += up(sizeof(int));
-  c.tileSum = o; o += up(kMaxTiles * sizeof(int));
-  c.cellCount = o; o += up(SG_NOALLOC_MAX_CELLS * sizeof(int));
   c.cellStart = o; o += up(SG_NOALLOC_MAX_CELLS * sizeof(int));
   c.cellOf = o; o += up(N * sizeof(int));
-  c.slot = o; o += up(N * sizeof(int));
-  c.tmpIdx = o; o += up(N * sizeof(int));
   c.sortIdx = o; o += up(N * sizeof(int));
   c.nn = o; o += up(N * sizeof(int));
   c.ns = o; o += up(N * sizeof(int));
@@ -73,8 +74,9 @@ constexpr Carve carve() {
   c.nrl = o; o += up(N * sizeof(int));
   c.rl = o; o += up(N * kRelMax * sizeof(unsigned));
   c.active = o; o += up(SG_NOALLOC_MAX_CELLS * sizeof(int));
-  c.heavy = o; o += up(((size_t)N / kHeavyChunk + (size_t)N / (kHeavyCell + 1) + 16) * sizeof(int2));
-  c.work = o; o += up(3 * sizeof(int));
+  // a cell of n > t atoms (t = kItem) gives ceil(n / t) items: at most N / t + N / (t + 1) in all
+  c.heavy = o; o += up(((size_t)N / kItem + (size_t)N / (kItem + 1) + 16) * sizeof(int2));
+  c.work = o; o += up(4 * sizeof(int));
   c.total = o;
   return c;
 }
@@ -89,29 +91,159 @@ constexpr int kMaxDevices = 64;
 unsigned char *g_base[kMaxDevices] = {};
 std::mutex g_mu;
 
-// Writes the parameter block, clears the state block and the cell counts, and fills the
-// block tables of a single system: everything that must start fresh on every call.
-__global__ void k_noalloc_setup(RepConst P, RepState *st, RepConst *rc, int *tabRep, int *tabStart,
-                                int *tileRep, int *tileStart, int *tileFirst, int *cellCount, int *work) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int stride = gridDim.x * blockDim.x;
-  if (t == 0) {
-    *rc = P;
-    memset(st, 0, sizeof(RepState));
-    st->nebrNow = 1;
-    *tileFirst = 0;
+// Block 0 writes the parameter block, clears the state block and the list build's counters, and fills
+// the block tables of a single system: everything that must start fresh on every call.  The others
+// find the cells of kSortThreads atoms each (-1: outside the grid; past the last atom one that no cell
+// has, up to a multiple of four).
+constexpr int kNoCell = 1 << 30;
+__global__ void __launch_bounds__(kSortThreads) k_noalloc_setup(const __grid_constant__ RepConst P, RepState *st,
+                                                                RepConst *rc, int *tabRep, int *tabStart, int *tileRep,
+                                                                int *work, const float4 *__restrict__ pos,
+                                                                int *__restrict__ cellOf, int *__restrict__ nn,
+                                                                int *__restrict__ ns, int *__restrict__ nrl) {
+  asm volatile("griddepcontrol.launch_dependents;");  // the sort's few blocks may take their places now
+  const int t = threadIdx.x, n = blockDim.x;
+  if (blockIdx.x > 0) {
+    const int g = (blockIdx.x - 1) * kSortThreads + t;
+    if (g < P.nMol) {
+      const float4 r = pos[g];
+      const int c = cellIndex(P, r.x, r.y, r.z);
+      cellOf[g] = c;
+      if (c < 0) nn[g] = ns[g] = nrl[g] = 0;  // no list (the reference clears its NN)
+    } else if (g < (P.nMol + 3 & ~3)) {
+      cellOf[g] = kNoCell;
+    }
+    return;
   }
-  for (int b = t; b < kMaxTabBlocks; b += stride) {
-    tabRep[b] = 0; tabStart[b] = b * kBs;                                   // atoms, 128 per block
-    tabRep[kMaxTabBlocks + b] = 0; tabStart[kMaxTabBlocks + b] = b * kMetalPerBlock;
-    tabRep[2 * kMaxTabBlocks + b] = 0; tabStart[2 * kMaxTabBlocks + b] = P.nMolMe + b * kCarbonPerBlock;
+  for (int q = t; q < (int)(sizeof(RepConst) / 4); q += n)
+    reinterpret_cast<int *>(rc)[q] = reinterpret_cast<const int *>(&P)[q];
+  for (int q = t; q < (int)(sizeof(RepState) / 4); q += n)
+    reinterpret_cast<int *>(st)[q] = q == (int)(offsetof(RepState, nebrNow) / 4) ? 1 : 0;
+  for (int b = t; b < 3 * kMaxTabBlocks; b += n) {
+    const int e = b % kMaxTabBlocks;
+    tabRep[b] = 0;
+    // atoms, 128 per block; metal atoms; carbon atoms
+    tabStart[b] = b < kMaxTabBlocks ? e * kBs : b < 2 * kMaxTabBlocks ? e * kMetalPerBlock : P.nMolMe + e * kCarbonPerBlock;
   }
-  for (int k = t; k < P.ncellsPad / kCellTile; k += stride) {
-    tileRep[k] = 0;
-    tileStart[k] = k * kCellTile;
+  if (t < kMaxTiles) tileRep[t] = 0;
+  if (t < 4) work[t] = 0;
+}
+
+// The atoms in cell order, ascending index inside a cell (sortIdx, sortPos), the cell starts and the
+// list build's work items, in one pass: a block per kSortCells cells looks at every atom's cell (at
+// most SG_NOALLOC_MAX_ATOMS, four of four a thread), counts those of earlier cells (its offset), keeps
+// its own in shared memory, groups them by cell there and ranks each among its cell's.  The passes it
+// replaces (count, three of a prefix sum, scatter, rank) were six launches of 3 to 9 us, each waiting
+// for the one before: 32 us of the 87 us of kernels of a 2,217-atom call, 35 of 107 us at 15,883 atoms;
+// now 8 and 12 us (ncu).  The whole call, with the two force passes in one launch and programmatic
+// dependent launch: 105 -> 55 us and 129 -> 67 us.
+// Dynamic shared memory: two words an atom.
+__global__ void __launch_bounds__(kSortThreads) k_noalloc_sort(int nMol, int ncells, RepState *st,
+                                                               const float4 *__restrict__ pos, const int *__restrict__ cellOf,
+                                                               int *__restrict__ cellStart, int cap,
+                                                               int2 *__restrict__ heavy, int *__restrict__ active,
+                                                               int *__restrict__ work, int *__restrict__ sortIdx,
+                                                               float4 *__restrict__ sortPos) {
+  extern __shared__ unsigned sAtoms[];  // {cell of the block << 15 | atom} as met, then by cell
+  __shared__ int sCount[kSortCells], sStart[kSortCells + 1], sBefore[kSortThreads / 32], sWarp[kSortCells / 32], sMine;
+  unsigned *met = sAtoms, *byCell = sAtoms + nMol;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, c0 = blockIdx.x * kSortCells;
+  if (tid < kSortCells) sCount[tid] = 0;
+  if (tid == 0) sMine = 0;
+  __syncthreads();
+  pdlEnter();
+  int before = 0, outside = 0;
+#pragma unroll 4
+  for (int q = tid; 4 * q < nMol; q += kSortThreads) {
+    const int4 v = reinterpret_cast<const int4 *>(cellOf)[q];
+    const int c[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      outside += c[u] < 0 ? 1 : 0;
+      before += c[u] >= 0 && c[u] < c0 ? 1 : 0;
+      if (c[u] >= c0 && c[u] < c0 + kSortCells) {
+        atomicAdd(&sCount[c[u] - c0], 1);
+        met[atomicAdd(&sMine, 1)] = (unsigned)(c[u] - c0) << 15 | (unsigned)(4 * q + u);
+      }
+    }
   }
-  for (int c = t; c < P.ncellsPad; c += stride) cellCount[c] = 0;
-  if (t < 3) work[t] = 0;
+  for (int o = 16; o > 0; o >>= 1) {
+    before += __shfl_xor_sync(0xffffffffu, before, o);
+    outside += __shfl_xor_sync(0xffffffffu, outside, o);
+  }
+  if (lane == 0) sBefore[wid] = before;
+  __syncthreads();
+  // prefix sum of the block's cells, a thread each
+  const int n = tid < kSortCells ? sCount[tid] : 0;
+  int incl = n;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  if (tid < kSortCells && lane == 31) sWarp[wid] = incl;
+  int base = sBefore[lane];  // kSortThreads / 32 = 32 warps
+  for (int o = 16; o > 0; o >>= 1) base += __shfl_xor_sync(0xffffffffu, base, o);
+  __syncthreads();
+  if (tid < kSortCells) {
+    int start = incl - n;
+    for (int q = 0; q < wid; q++) start += sWarp[q];
+    sStart[tid] = start;
+    if (tid == kSortCells - 1) sStart[kSortCells] = start + n;
+    if (c0 + tid <= ncells) cellStart[c0 + tid] = base + start;
+    sCount[tid] = 0;  // arrivals of the grouping below
+  }
+  __syncthreads();
+  // the work items: places in the lists asked for now, used at the end
+  const bool live = n > 0 && c0 + tid < ncells;
+  const int nHeavy = live && n > kItem ? (n + kItem - 1) / kItem : 0, nLight = live && n <= kItem ? 1 : 0;
+  int preH = nHeavy, preL = nLight, occ = n, over = n > cap ? 1 : 0, atH = 0, atL = 0;
+  if (tid < kSortCells) {
+    for (int o = 1; o < 32; o <<= 1) {
+      const int yh = __shfl_up_sync(0xffffffffu, preH, o), yl = __shfl_up_sync(0xffffffffu, preL, o);
+      if (lane >= o) {
+        preH += yh;
+        preL += yl;
+      }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      occ = max(occ, __shfl_xor_sync(0xffffffffu, occ, o));
+      over += __shfl_xor_sync(0xffffffffu, over, o);
+    }
+    if (lane == 31) {
+      if (preL) atL = atomicAdd(&work[1], preL);
+      if (preH) atH = atomicAdd(&work[2], preH);
+      if (occ) atomicMax(&st->maxCellOcc, occ);
+      if (over) {
+        atomicAdd(&st->cellOverflow, over);
+        setFlag(st, 11 /*SG_ERR_CELL_OVERFLOW*/);
+      }
+    }
+  }
+  if (blockIdx.x == 0 && lane == 0 && outside) atomicAdd(&st->cellRange, outside);
+  const int mine = sMine;
+  for (int q = tid; q < mine; q += kSortThreads) {
+    const unsigned v = met[q];
+    byCell[sStart[v >> 15] + atomicAdd(&sCount[v >> 15], 1)] = v;
+  }
+  __syncthreads();
+  for (int q = tid; q < mine; q += kSortThreads) {
+    const unsigned v = byCell[q];
+    const int c = v >> 15, g = v & 0x7fff, b = sStart[c], e = sStart[c + 1];
+    float4 r = pos[g];
+    int rank = 0;
+    for (int k = b; k < e; k++) rank += byCell[k] < v ? 1 : 0;  // the same cell: compares atoms
+    r.w = __int_as_float(g);
+    sortIdx[base + b + rank] = g;
+    sortPos[base + b + rank] = r;
+  }
+  if (tid >= kSortCells) return;
+  atH = __shfl_sync(0xffffffffu, atH, 31) + preH - nHeavy;
+  atL = __shfl_sync(0xffffffffu, atL, 31) + preL - nLight;
+  for (int j = 0; j < nHeavy; j++) {
+    const int h0 = j * n / nHeavy, h1 = (j + 1) * n / nHeavy;
+    heavy[atH + j] = make_int2(c0 + tid, h0 << 16 | (h1 - h0));
+  }
+  if (nLight) active[atL] = c0 + tid;
 }
 
 RepConst constFor(const sg_simparams &p) {
@@ -154,7 +286,6 @@ extern "C" int sg_compute_forces_noalloc(const sg_simparams *p, sg_float4 *d_pos
                    "sg_compute_forces_noalloc: system exceeds the static scratch (nMol %d of max %d, "
                    "padded cells %lld of max %d, iNebrMax %d of max %d)",
                    p->nMol, SG_NOALLOC_MAX_ATOMS, ncellsPad64, SG_NOALLOC_MAX_CELLS, p->iNebrMax, SG_NOALLOC_MAX_NEBR);
-  const int ncellsPad = (int)ncellsPad64;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess || dev < 0 || dev >= kMaxDevices)
@@ -167,6 +298,11 @@ extern "C" int sg_compute_forces_noalloc(const sg_simparams *p, sg_float4 *d_pos
       e = cudaGetSymbolAddress(&ptr, g_scratch);
       if (e != cudaSuccess)
         return sg_fail(SG_ERR_CUDA, "cudaGetSymbolAddress(scratch): %s", cudaGetErrorString(e));
+      // the sort's shared memory at the largest system
+      e = cudaFuncSetAttribute(k_noalloc_sort, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)(2 * sizeof(unsigned) * SG_NOALLOC_MAX_ATOMS));
+      if (e != cudaSuccess)
+        return sg_fail(SG_ERR_CUDA, "cudaFuncSetAttribute(k_noalloc_sort): %s", cudaGetErrorString(e));
       g_base[dev] = (unsigned char *)ptr;
     }
     base = g_base[dev];
@@ -176,11 +312,8 @@ extern "C" int sg_compute_forces_noalloc(const sg_simparams *p, sg_float4 *d_pos
   RepConst *rc = (RepConst *)(base + K.rc);
   RepState *st = (RepState *)(base + K.st);
   int *tabRep = (int *)(base + K.tabRep), *tabStart = (int *)(base + K.tabStart);
-  int *tileRep = (int *)(base + K.tileRep), *tileStart = (int *)(base + K.tileStart);
-  int *tileFirst = (int *)(base + K.tileFirst), *tileSum = (int *)(base + K.tileSum);
-  int *cellCount = (int *)(base + K.cellCount), *cellStart = (int *)(base + K.cellStart);
-  int *cellOf = (int *)(base + K.cellOf), *slot = (int *)(base + K.slot), *tmpIdx = (int *)(base + K.tmpIdx);
-  int *sortIdx = (int *)(base + K.sortIdx), *nn = (int *)(base + K.nn), *ns = (int *)(base + K.ns);
+  int *tileRep = (int *)(base + K.tileRep), *cellStart = (int *)(base + K.cellStart);
+  int *cellOf = (int *)(base + K.cellOf), *sortIdx = (int *)(base + K.sortIdx), *nn = (int *)(base + K.nn), *ns = (int *)(base + K.ns);
   int *sl = (int *)(base + K.sl);
   float4 *sortPos = (float4 *)(base + K.sortPos);
   float *rho = (float *)(base + K.rho), *dF = (float *)(base + K.dF), *Fv = (float *)(base + K.Fv);
@@ -193,33 +326,23 @@ extern "C" int sg_compute_forces_noalloc(const sg_simparams *p, sg_float4 *d_pos
 
   const RepConst P = constFor(*p);
   const int N = p->nMol;
-  const int nAtomBlk = (N + kBs - 1) / kBs;
   const int nMetalBlk = (p->nMolMe + kMetalPerBlock - 1) / kMetalPerBlock;
   const int nCarbBlk = (N - p->nMolMe + kCarbonPerBlock - 1) / kCarbonPerBlock;
-  const int nTiles = ncellsPad / kCellTile;
-  BlockTab atomTab{tabRep, tabStart, nAtomBlk};
   BlockTab metalTab{tabRep + kMaxTabBlocks, tabStart + kMaxTabBlocks, nMetalBlk};
   BlockTab carbTab{tabRep + 2 * kMaxTabBlocks, tabStart + 2 * kMaxTabBlocks, nCarbBlk};
-  BlockTab tileTab{tileRep, tileStart, nTiles};
-
-
-  k_noalloc_setup<<<64, 256, 0, s>>>(P, st, rc, tabRep, tabStart, tileRep, tileStart, tileFirst, cellCount, work);
-  k_cell_count<<<nAtomBlk, kBs, 0, s>>>(atomTab, rc, pos, cellOf, slot, cellCount);
-  k_scan_tiles<<<nTiles, 256, 0, s>>>(tileTab, rc, st, cellCount, tileSum, 1);
-  k_scan_tile_prefix<<<1, 1024, 0, s>>>(rc, st, tileFirst, tileSum, 1, nullptr);
-  k_scan_final<<<nTiles, 256, 0, s>>>(tileTab, rc, st, cellCount, tileSum, cellStart, (int)p->blockSize, 1, active,
-                                      heavy, work, kHeavyCell);
-  k_scatter<<<nAtomBlk, kBs, 0, s>>>(atomTab, rc, st, cellOf, slot, cellStart, tmpIdx, nn, ns, nrl, 1);
-  k_rank<<<nAtomBlk, kBs, 0, s>>>(atomTab, rc, st, cellOf, cellStart, tmpIdx, pos, sortIdx, sortPos, 1);
   const int rowStride = (p->iNebrMax + 3) & ~3;
-  k_build_nebr<<<256, kNebrWarps * 32, 0, s>>>(tileRep, active, heavy, work, rc, st, cellStart, sortPos, nn, nbl, ns,
-                                               sl, nrl, rl, rowStride, p->iNebrMax, 0,
-                                               nullptr, 0);
-  if (nMetalBlk) {
-    k_rho<<<nMetalBlk, kBs, 0, s>>>(metalTab, rc, pos, nn, nbl, rho, dF, Fv, rowStride);
-    k_force_metal<<<nMetalBlk, kBs, 0, s>>>(metalTab, rc, pos, acc, nn, nbl, dF, Fv, fric, rowStride);
-  }
-  if (nCarbBlk) launchCarbon(false, 8, nCarbBlk, s, carbTab, rc, pos, acc, nn, nbl, ns, sl, nrl, rl, rowStride);
+  const size_t sortSmem = 2 * sizeof(unsigned) * N;
+
+  k_noalloc_setup<<<1 + (N + kSortThreads + 3) / kSortThreads, kSortThreads, 0, s>>>(P, st, rc, tabRep, tabStart, tileRep, work,
+                                                                                     pos, cellOf, nn, ns, nrl);
+  launchK(true, k_noalloc_sort, P.ncells / kSortCells + 1, kSortThreads, sortSmem, s, N, P.ncells, st, pos, cellOf, cellStart,
+          (int)p->blockSize, heavy, active, work, sortIdx, sortPos);
+  launchK(true, k_build_nebr, kBuildBlocks, kNebrWarps * 32, 0, s, tileRep, active, heavy, work, rc, st, cellStart, sortPos, nn,
+          nbl, ns, sl, nrl, rl, rowStride, p->iNebrMax, 0, nullptr, 0);
+  if (nMetalBlk)
+    launchK(true, k_rho, nMetalBlk, kBs, 0, s, metalTab, rc, pos, nn, nbl, rho, dF, Fv, rowStride);
+  launchK(true, k_force_both, nMetalBlk + nCarbBlk, kBs, 0, s, metalTab, carbTab, rc, pos, acc, nn, nbl, ns, sl, nrl, rl, dF, Fv,
+          fric, rowStride);
   e = cudaGetLastError();
   if (e != cudaSuccess) return sg_fail(SG_ERR_CUDA, "sg_compute_forces_noalloc launch: %s", cudaGetErrorString(e));
   int flags = 0;
