@@ -728,15 +728,27 @@ static int enqueueRdf(sg_ctx *c, bool zero) {
     if (c->histExt)
       CK(cudaMemsetAsync(c->histExt, 0, sizeof(unsigned long long) * c->nrep * c->opt.rdf_ext_bins, c->stream));
   }
-  if (c->rdfTab.n && c->maxHist > 0) {
+  // the two samples side by side: neither fills the GPU (inside a capture the fork and join become
+  // graph edges)
+  const bool stencil = c->rdfTab.n && c->maxHist > 0, ext = c->histExt && c->nRdfPairs, fork = stencil && ext;
+  if (fork) {
+    CK(cudaEventRecord(c->evFork, c->stream));
+    CK(cudaStreamWaitEvent(c->side, c->evFork, 0));
+  }
+  if (stencil) {
     CK(launchK(c->pdl, k_rdf, c->rdfTab.n, 32 * kRdfAtoms, c->maxHist * sizeof(unsigned), c->stream,
                c->rdfTab.view(), c->rc, c->st, c->pos, c->cellOf, c->cellStart, c->sortIdx, c->hist, c->histStride));
     LAUNCH_OK();
   }
-  if (c->histExt && c->nRdfPairs) {
-    CK(launchK(c->pdl, k_rdf_ext, c->nRdfPairs, kRdfTile, c->opt.rdf_ext_bins * sizeof(unsigned), c->stream,
-               c->rc, c->pos, c->rdfPairs, c->histExt, c->opt.rdf_ext_bins, c->opt.rdf_ext_range));
+  if (ext) {
+    CK(launchK(c->pdl, k_rdf_ext, c->nRdfPairs, kRdfTile * kRdfGroups, c->opt.rdf_ext_bins * sizeof(unsigned),
+               fork ? c->side : c->stream, c->rc, c->pos, c->rdfPairs, c->histExt, c->opt.rdf_ext_bins,
+               c->opt.rdf_ext_range));
     LAUNCH_OK();
+  }
+  if (fork) {
+    CK(cudaEventRecord(c->evJoin, c->side));
+    CK(cudaStreamWaitEvent(c->stream, c->evJoin, 0));
   }
   return SG_OK;
 }
