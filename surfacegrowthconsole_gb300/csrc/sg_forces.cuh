@@ -216,7 +216,7 @@ __device__ __forceinline__ void SG_KN(rhoBody)(int e, const RepConst &P, BlockTa
     const int n = nn[i];
     const int *row = nbl + (size_t)i * rowStride;
     // kMetalBatch entries per lane per round: their indices, then their positions, load
-    // together (the sum still takes the entries in the same order)
+    // together; their densities are added in pairs (fewer roundings in sequence)
     for (int j0 = sub; j0 < n; j0 += kMetalBatch * MT) {
       int k[kMetalBatch];
       float4 B[kMetalBatch];
@@ -224,6 +224,7 @@ __device__ __forceinline__ void SG_KN(rhoBody)(int e, const RepConst &P, BlockTa
       for (int q = 0; q < kMetalBatch; q++) k[q] = (j0 + q * MT < n) ? row[j0 + q * MT] : -1;
 #pragma unroll
       for (int q = 0; q < kMetalBatch; q++) B[q] = (k[q] >= 0) ? pos[k[q]] : A;
+      float d[kMetalBatch] = {};
 #pragma unroll
       for (int q = 0; q < kMetalBatch; q++) {
         if (k[q] < 0) continue;
@@ -232,11 +233,12 @@ __device__ __forceinline__ void SG_KN(rhoBody)(int e, const RepConst &P, BlockTa
         const float dz = minImg(A.z - B[q].z, P.region[2]);
         const float rr = dx * dx + dy * dy + dz * dz;
 #ifdef SG_FAST_RECIP
-        if ((rr < P.rrCutEam) && (k[q] < metalEnd)) sum += SG_EAM_DENS(P, rr * rsqrtf(rr));
+        if ((rr < P.rrCutEam) && (k[q] < metalEnd)) d[q] = SG_EAM_DENS(P, rr * rsqrtf(rr));
 #else
-        if ((rr < P.rrCutEam) && (k[q] < metalEnd)) sum += SG_EAM_DENS(P, sqrtf(rr));
+        if ((rr < P.rrCutEam) && (k[q] < metalEnd)) d[q] = SG_EAM_DENS(P, sqrtf(rr));
 #endif
       }
+      sum += (d[0] + d[1]) + (d[2] + d[3]);
     }
   }
 #pragma unroll
