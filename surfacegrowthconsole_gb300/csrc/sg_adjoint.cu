@@ -1117,6 +1117,7 @@ extern "C" int sg_diff_forces(sg_diff *d, const double *theta, float *out) {
   DCK(cudaMemsetAsync(c->stage, 0, sizeof(float) * 3 * d->n, c->stream));  // atoms without a pair
   if (int rc = uploadModel(d, theta)) return rc;
   if (int rc = forces(d, c->stage, nullptr, 0.f, 0, false)) return rc;
+  sg_populate(out, sizeof(float) * 3 * d->n);  // while the passes run
   DCK(cudaMemcpyAsync(out, c->stage, sizeof(float) * 3 * d->n, cudaMemcpyDeviceToHost, c->stream));
   DCK(cudaStreamSynchronize(c->stream));
   return SG_OK;

@@ -11,8 +11,11 @@
 // one graph launch and no host synchronisation; the host reads results only at output
 // points.
 #include <cuda_runtime.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <algorithm>
+#include <cerrno>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -582,6 +585,23 @@ static int download3(sg_ctx *c, const float4 *d, sg_float3 *h, int n) {
   return SG_OK;
 }
 
+// The pages of a host array about to be written by the device, made present.  A page that the process
+// has not touched yet costs the device about 19 us to fault in (64 KB; 716,263 atoms' state, 28 MB,
+// took 7.5 to 8.6 ms), the process 2 us, and a present one next to nothing (5 us for 1.8 MB).  Below
+// 128 KB allocators hand out memory in use.  A kernel or mapping that cannot do it leaves it to the
+// device.
+void sg_populate(void *p, size_t bytes) {
+#ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_WRITE 23
+#endif
+  if (!p || bytes < (128u << 10)) return;
+  const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), a = reinterpret_cast<uintptr_t>(p) & ~(page - 1);
+  const int keep = errno;
+  (void)madvise(reinterpret_cast<void *>(a), (reinterpret_cast<uintptr_t>(p) + bytes - a + page - 1) & ~(page - 1),
+                MADV_POPULATE_WRITE);
+  errno = keep;
+}
+
 // The device address of a host array the GPU can read in place (page-locked, mapped into the
 // unified address space: cudaMallocHost, cudaHostAlloc, cudaHostRegister), else nullptr.
 static const void *mappedHost(const void *h) {
@@ -657,6 +677,26 @@ extern "C" int sg_get_state(sg_ctx *c, int rep, sg_float4 *r, sg_float3 *v, sg_f
   if (!c) return sg_fail(SG_ERR_INVALID, "null context");
   int off, n, rc;
   if ((rc = repRange(c, rep, off, n))) return rc;
+  if (c->hostDirect && (reinterpret_cast<uintptr_t>(r) & 15) == 0) {
+    // one launch writes the caller's arrays in place, whatever their allocation, and one wait (the
+    // route below is six operations and up to three waits: 45,546 atoms into fresh pages 110 us, 72 here)
+    if (!r && !v && !a) return SG_OK;
+    sg_populate(r, (size_t)n * sizeof(*r));
+    sg_populate(v, (size_t)n * sizeof(*v));
+    sg_populate(a, (size_t)n * sizeof(*a));
+    BlockTab tab = c->atomTab.view();
+    if (rep >= 0) {  // the replica's entries: the table lists the replicas in order
+      int first = 0;
+      for (int q = 0; q < rep; q++) first += (c->hrc[q].nMol + 127) / 128;
+      tab = BlockTab{tab.rep + first, tab.start + first, (n + 127) / 128};
+    }
+    k_read_state<<<tab.nblocks, 128, 0, c->stream>>>(tab, c->rc, c->st, c->pos, c->vel, c->acc, off,
+                                                     reinterpret_cast<float4 *>(r), reinterpret_cast<float *>(v),
+                                                     reinterpret_cast<float *>(a));
+    CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(c->stream));
+    return SG_OK;
+  }
   if (v && (rc = applyPending(c))) return rc;
   if (r) CK(cudaMemcpyAsync(r, c->pos + off, (size_t)n * sizeof(float4), cudaMemcpyDeviceToHost, c->stream));
   if (v && (rc = download3(c, c->vel + off, v, n))) return rc;

@@ -116,6 +116,7 @@ struct sg_ctx {
 
 int sg_fail(int code, const char *fmt, ...);
 
+void sg_populate(void *p, size_t bytes);
 int sg_read_state(sg_ctx *c, int rep, sg::RepState *out);
 int sg_get_diffusion_print(sg_ctx *c, int rep, float *table, int *nprints);
 int sg_next_variant(sg_ctx *c);
