@@ -19,7 +19,8 @@
 //                                           one word (relPack)
 //   ns int[Ntot], sl int[Ntot * kShortMax]  close list of a carbon atom: its entries within
 //                                           (rCutC+skin), in list order
-//   rho/dF/Fv float[Ntot]   EAM density, F'(rho), F(rho) (metal atoms)
+//   rho/Fv float[Ntot]     EAM density, F(rho) (metal atoms)
+//   posF float4[Ntot]      x, y, z, F'(rho) of the metal atoms, written by the density pass
 //   fric float[Ntot]       x force of carbon on each metal atom
 // Per-replica constants live in RepConst, mutable per-replica scalars in RepState.
 #pragma once

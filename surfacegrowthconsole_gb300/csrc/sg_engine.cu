@@ -372,7 +372,7 @@ extern "C" int sg_create(const sg_simparams *params, int n_replicas, const sg_op
   AL(c->nebrWork, 4);  // next item, light items, heavy items, spill-list length
   if (c->opt.mode == SG_MODE_MIXED) AL(c->spill, std::max<size_t>(N, 1));
   AL(c->bucket, (size_t)c->ctot * c->bucketCap);
-  AL(c->rho, N); AL(c->dF, N); AL(c->Fv, N); AL(c->fric, N);
+  AL(c->rho, N); AL(c->posF, N); AL(c->Fv, N); AL(c->fric, N);
   AL(c->partial, (size_t)std::max(redOff, 1) * kNumRed);
   AL(c->partialCmv, (size_t)std::max(cmvOff, 1) * 3);
   AL(c->dRedFirst, n_replicas); AL(c->dCmvFirst, n_replicas);
@@ -741,7 +741,7 @@ static int enqueueForces(sg_ctx *c, bool withCmVel) {
     CK(cudaEventRecord(c->evFork, c->stream));
     CK(cudaStreamWaitEvent(c->side, c->evFork, 0));
     launchMetalChain(c->pdl, c->metalLanes, c->metalRun.n, 0, 0, c->side, c->metalRun.view(), c->rc, c->pos, c->acc, c->nn,
-                     c->nbl, c->rho, c->dF, c->Fv, c->fric, c->rowStride);
+                     c->nbl, c->rho, c->posF, c->Fv, c->fric, c->rowStride);
     if (withCmVel && c->cmvTab.n)
       CK(launchK(c->pdl, k_cmvel, c->cmvTab.n, kRedThreads, 0, c->side, c->cmvTab.view(), c->rc, c->st, c->vel, c->acc,
                                                         c->partialCmv, c->dCmvFirst));

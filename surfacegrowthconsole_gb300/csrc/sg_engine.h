@@ -56,7 +56,8 @@ struct sg_ctx {
   int scanCells = sg::kScanCells;  // cells per block of the scan and ordering
   int nScanBlocks = 0;
   int2 *heavyItems = nullptr;
-  float *rho = nullptr, *dF = nullptr, *Fv = nullptr, *fric = nullptr;
+  float *rho = nullptr, *Fv = nullptr, *fric = nullptr;
+  float4 *posF = nullptr;
   float *partial = nullptr, *partialCmv = nullptr;
   int *dRedFirst = nullptr, *dCmvFirst = nullptr, *dTileFirst = nullptr;
   unsigned *hist = nullptr;

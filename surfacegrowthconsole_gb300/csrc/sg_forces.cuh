@@ -192,7 +192,8 @@ __device__ __forceinline__ float eamDensTab(const RepConst &P, const float4 *tab
 // Electron density of each metal atom (EamComputeRhoK, cu:716-773), plus F(rho) and F'(rho),
 // which the reference re-evaluates per pair in the force kernel.  MT lanes share one metal
 // atom (128 / MT atoms per block): lane l takes list entries l, l + MT, ...; the partial sums
-// meet in a shuffle tree.  k_rho runs MT = kMT; k_rho_tpa<MT> the choices of the autotuner.
+// meet in a shuffle tree.  F' goes out as the fourth word of a copy of the atom's position (posF), so
+// that the force pass, which is bound by its gathers, has one per metal entry instead of two.  k_rho runs MT = kMT; k_rho_tpa<MT> the choices of the autotuner.
 constexpr int kMetalBatch = 4;  // list entries per lane whose loads are issued together
 template <int MT> __device__ __forceinline__ unsigned laneGroupMask() {
   return MT == 32 ? 0xffffffffu : ((1u << MT) - 1) << (threadIdx.x & 31 & ~(MT - 1));
@@ -203,7 +204,7 @@ template <int MT>
 __device__ __forceinline__ void SG_KN(rhoBody)(int e, const RepConst &P, BlockTab tab,
                                                const float4 *__restrict__ pos, const int *__restrict__ nn,
                                                const int *__restrict__ nbl, float *__restrict__ rho,
-                                               float *__restrict__ dF, float *__restrict__ Fv,
+                                               float4 *__restrict__ posF, float *__restrict__ Fv,
                                                int rowStride SG_EAM_BODY_PARAM) {
   const int sub = threadIdx.x & (MT - 1);
   const unsigned gmask = laneGroupMask<MT>();
@@ -211,8 +212,9 @@ __device__ __forceinline__ void SG_KN(rhoBody)(int e, const RepConst &P, BlockTa
   const int metalEnd = P.atomOff + P.nMolMe;
   const bool valid = i < metalEnd;
   float sum = 0.f;
+  float4 A = make_float4(0.f, 0.f, 0.f, 0.f);
   if (valid) {
-    const float4 A = pos[i];
+    A = pos[i];
     const int n = nn[i];
     const int *row = nbl + (size_t)i * rowStride;
     // kMetalBatch entries per lane per round: their indices, then their positions, load
@@ -245,7 +247,7 @@ __device__ __forceinline__ void SG_KN(rhoBody)(int e, const RepConst &P, BlockTa
   for (int o = MT / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(gmask, sum, o);
   if (valid && sub == 0) {
     rho[i] = sum;
-    dF[i] = eamEmbedDeriv(P, sum);
+    posF[i] = make_float4(A.x, A.y, A.z, eamEmbedDeriv(P, sum));
     Fv[i] = eamEmbed(P, sum);
   }
 }
@@ -253,21 +255,21 @@ __device__ __forceinline__ void SG_KN(rhoBody)(int e, const RepConst &P, BlockTa
 __global__ void __launch_bounds__(128) SG_KN(k_rho)(BlockTab tab, const RepConst *__restrict__ rc,
                                              const float4 *__restrict__ pos, const int *__restrict__ nn,
                                              const int *__restrict__ nbl, float *__restrict__ rho,
-                                             float *__restrict__ dF, float *__restrict__ Fv,
+                                             float4 *__restrict__ posF, float *__restrict__ Fv,
                                              int rowStride SG_EAM_PARAM) {
   pdlEnter();
   const RepConst &P = rc[tab.rep[blockIdx.x]];
-  SG_KN(rhoBody)<kMT>(blockIdx.x, P, tab, pos, nn, nbl, rho, dF, Fv, rowStride SG_EAM_BASE(P));
+  SG_KN(rhoBody)<kMT>(blockIdx.x, P, tab, pos, nn, nbl, rho, posF, Fv, rowStride SG_EAM_BASE(P));
 }
 template <int MT>
 __global__ void __launch_bounds__(128) SG_KN(k_rho_tpa)(BlockTab tab, const RepConst *__restrict__ rc,
                                                  const float4 *__restrict__ pos, const int *__restrict__ nn,
                                                  const int *__restrict__ nbl, float *__restrict__ rho,
-                                                 float *__restrict__ dF, float *__restrict__ Fv,
+                                                 float4 *__restrict__ posF, float *__restrict__ Fv,
                                                  int rowStride SG_EAM_PARAM) {
   pdlEnter();
   const RepConst &P = rc[tab.rep[blockIdx.x]];
-  SG_KN(rhoBody)<MT>(blockIdx.x, P, tab, pos, nn, nbl, rho, dF, Fv, rowStride SG_EAM_BASE(P));
+  SG_KN(rhoBody)<MT>(blockIdx.x, P, tab, pos, nn, nbl, rho, posF, Fv, rowStride SG_EAM_BASE(P));
 }
 
 // Lennard-Jones metal-carbon term (cu:880-884).
@@ -292,7 +294,7 @@ template <int MT>
 __device__ __forceinline__ void SG_KN(forceMetalBody)(int e, const RepConst &P, BlockTab tab,
                                                       float4 *__restrict__ pos, float4 *__restrict__ acc,
                                                       const int *__restrict__ nn, const int *__restrict__ nbl,
-                                                      const float *__restrict__ dF,
+                                                      const float4 *__restrict__ posF,
                                                       const float *__restrict__ Fv, float *__restrict__ fric,
                                                       int rowStride SG_EAM_BODY_PARAM) {
   const int sub = threadIdx.x & (MT - 1);
@@ -302,22 +304,18 @@ __device__ __forceinline__ void SG_KN(forceMetalBody)(int e, const RepConst &P, 
   const bool valid = i < metalEnd;
   float fx = 0.f, fy = 0.f, fz = 0.f, rx = 0.f, u = 0.f;
   if (valid) {
-    const float4 A = pos[i];
+    const float4 A = posF[i];
     const int n = nn[i];
-    const float dFi = dF[i];
+    const float dFi = A.w;
     const int *row = nbl + (size_t)i * rowStride;
     // batches of entries as in the density pass; same order of the sums
     for (int j0 = sub; j0 < n; j0 += kMetalBatch * MT) {
       int k[kMetalBatch];
       float4 B[kMetalBatch];
-      float dFk[kMetalBatch];
 #pragma unroll
       for (int q = 0; q < kMetalBatch; q++) k[q] = (j0 + q * MT < n) ? row[j0 + q * MT] : -1;
 #pragma unroll
-      for (int q = 0; q < kMetalBatch; q++) {
-        B[q] = (k[q] >= 0) ? pos[k[q]] : A;
-        dFk[q] = (k[q] >= 0 && k[q] < metalEnd) ? dF[k[q]] : 0.f;
-      }
+      for (int q = 0; q < kMetalBatch; q++) B[q] = (k[q] >= 0) ? (k[q] < metalEnd ? posF : pos)[k[q]] : A;
 #pragma unroll
       for (int q = 0; q < kMetalBatch; q++) {
         if (k[q] < 0) continue;
@@ -335,7 +333,7 @@ __device__ __forceinline__ void SG_KN(forceMetalBody)(int e, const RepConst &P, 
 #endif
           const EamPair e = SG_EAM_PAIR(P, r);
           float fc = -e.dphi;
-          fc = fc - e.df * (dFi + dFk[q]);
+          fc = fc - e.df * (dFi + B[q].w);
 #ifdef SG_FAST_RECIP
           fc = fc * ri;
 #else
@@ -372,22 +370,22 @@ __device__ __forceinline__ void SG_KN(forceMetalBody)(int e, const RepConst &P, 
 __global__ void __launch_bounds__(128) SG_KN(k_force_metal)(BlockTab tab, const RepConst *__restrict__ rc,
                                                      float4 *__restrict__ pos, float4 *__restrict__ acc,
                                                      const int *__restrict__ nn, const int *__restrict__ nbl,
-                                                     const float *__restrict__ dF, const float *__restrict__ Fv,
+                                                     const float4 *__restrict__ posF, const float *__restrict__ Fv,
                                                      float *__restrict__ fric, int rowStride SG_EAM_PARAM) {
   pdlEnter();
   const RepConst &P = rc[tab.rep[blockIdx.x]];
-  SG_KN(forceMetalBody)<kMT>(blockIdx.x, P, tab, pos, acc, nn, nbl, dF, Fv, fric, rowStride SG_EAM_BASE(P));
+  SG_KN(forceMetalBody)<kMT>(blockIdx.x, P, tab, pos, acc, nn, nbl, posF, Fv, fric, rowStride SG_EAM_BASE(P));
 }
 template <int MT>
 __global__ void __launch_bounds__(128) SG_KN(k_force_metal_tpa)(BlockTab tab, const RepConst *__restrict__ rc,
                                                          float4 *__restrict__ pos, float4 *__restrict__ acc,
                                                          const int *__restrict__ nn, const int *__restrict__ nbl,
-                                                         const float *__restrict__ dF,
+                                                         const float4 *__restrict__ posF,
                                                          const float *__restrict__ Fv, float *__restrict__ fric,
                                                          int rowStride SG_EAM_PARAM) {
   pdlEnter();
   const RepConst &P = rc[tab.rep[blockIdx.x]];
-  SG_KN(forceMetalBody)<MT>(blockIdx.x, P, tab, pos, acc, nn, nbl, dF, Fv, fric, rowStride SG_EAM_BASE(P));
+  SG_KN(forceMetalBody)<MT>(blockIdx.x, P, tab, pos, acc, nn, nbl, posF, Fv, fric, rowStride SG_EAM_BASE(P));
 }
 
 #ifdef SG_EAM_TABLE
@@ -398,7 +396,7 @@ template <int MT>
 __global__ void __launch_bounds__(128) SG_KN(k_rho_staged)(BlockTab tab, const RepConst *__restrict__ rc,
                                                     const float4 *__restrict__ pos, const int *__restrict__ nn,
                                                     const int *__restrict__ nbl, float *__restrict__ rho,
-                                                    float *__restrict__ dF, float *__restrict__ Fv,
+                                                    float4 *__restrict__ posF, float *__restrict__ Fv,
                                                     int rowStride SG_EAM_PARAM) {
   extern __shared__ float4 sTab[];
   pdlEnter();
@@ -412,14 +410,14 @@ __global__ void __launch_bounds__(128) SG_KN(k_rho_staged)(BlockTab tab, const R
       __syncthreads();
       staged = rep;
     }
-    SG_KN(rhoBody)<MT>(e, P, tab, pos, nn, nbl, rho, dF, Fv, rowStride, sTab);
+    SG_KN(rhoBody)<MT>(e, P, tab, pos, nn, nbl, rho, posF, Fv, rowStride, sTab);
   }
 }
 template <int MT>
 __global__ void __launch_bounds__(128) SG_KN(k_force_metal_staged)(BlockTab tab, const RepConst *__restrict__ rc,
                                                             float4 *__restrict__ pos, float4 *__restrict__ acc,
                                                             const int *__restrict__ nn, const int *__restrict__ nbl,
-                                                            const float *__restrict__ dF,
+                                                            const float4 *__restrict__ posF,
                                                             const float *__restrict__ Fv,
                                                             float *__restrict__ fric, int rowStride SG_EAM_PARAM) {
   extern __shared__ float4 sTab[];
@@ -434,16 +432,16 @@ __global__ void __launch_bounds__(128) SG_KN(k_force_metal_staged)(BlockTab tab,
       __syncthreads();
       staged = rep;
     }
-    SG_KN(forceMetalBody)<MT>(e, P, tab, pos, acc, nn, nbl, dF, Fv, fric, rowStride, sTab);
+    SG_KN(forceMetalBody)<MT>(e, P, tab, pos, acc, nn, nbl, posF, Fv, fric, rowStride, sTab);
   }
 }
 
 template <int MT>
 static void SG_KN(launchStaged)(bool pdl, int grid, size_t smem, cudaStream_t s, BlockTab tab, const RepConst *rc,
-                                float4 *pos, float4 *acc, const int *nn, const int *nbl, float *rho, float *dF,
+                                float4 *pos, float4 *acc, const int *nn, const int *nbl, float *rho, float4 *posF,
                                 float *Fv, float *fric, int rowStride, const float4 *eamTab) {
-  launchK(pdl, SG_KN(k_rho_staged)<MT>, grid, 128, smem, s, tab, rc, pos, nn, nbl, rho, dF, Fv, rowStride, eamTab);
-  launchK(pdl, SG_KN(k_force_metal_staged)<MT>, grid, 128, smem, s, tab, rc, pos, acc, nn, nbl, dF, Fv, fric,
+  launchK(pdl, SG_KN(k_rho_staged)<MT>, grid, 128, smem, s, tab, rc, pos, nn, nbl, rho, posF, Fv, rowStride, eamTab);
+  launchK(pdl, SG_KN(k_force_metal_staged)<MT>, grid, 128, smem, s, tab, rc, pos, acc, nn, nbl, posF, Fv, fric,
           rowStride, eamTab);
 }
 #endif
@@ -454,16 +452,16 @@ static void SG_KN(launchStaged)(bool pdl, int grid, size_t smem, cudaStream_t s,
 // with stagedSmem bytes of table (launch errors are left for cudaGetLastError).
 void SG_KN(launchMetalChain)(bool pdl, int mt, int grid, int stagedGrid, size_t stagedSmem, cudaStream_t s,
                              BlockTab tab, const RepConst *rc, float4 *pos, float4 *acc, const int *nn,
-                             const int *nbl, float *rho, float *dF, float *Fv, float *fric,
+                             const int *nbl, float *rho, float4 *posF, float *Fv, float *fric,
                              int rowStride SG_EAM_PARAM) {
 #ifdef SG_EAM_TABLE
   if (stagedGrid > 0) {
     const int g = grid < stagedGrid ? grid : stagedGrid;
     switch (mt) {
-      case 4: SG_KN(launchStaged)<4>(pdl, g, stagedSmem, s, tab, rc, pos, acc, nn, nbl, rho, dF, Fv, fric, rowStride, eamTab); break;
-      case 8: SG_KN(launchStaged)<8>(pdl, g, stagedSmem, s, tab, rc, pos, acc, nn, nbl, rho, dF, Fv, fric, rowStride, eamTab); break;
-      case 32: SG_KN(launchStaged)<32>(pdl, g, stagedSmem, s, tab, rc, pos, acc, nn, nbl, rho, dF, Fv, fric, rowStride, eamTab); break;
-      default: SG_KN(launchStaged)<16>(pdl, g, stagedSmem, s, tab, rc, pos, acc, nn, nbl, rho, dF, Fv, fric, rowStride, eamTab);
+      case 4: SG_KN(launchStaged)<4>(pdl, g, stagedSmem, s, tab, rc, pos, acc, nn, nbl, rho, posF, Fv, fric, rowStride, eamTab); break;
+      case 8: SG_KN(launchStaged)<8>(pdl, g, stagedSmem, s, tab, rc, pos, acc, nn, nbl, rho, posF, Fv, fric, rowStride, eamTab); break;
+      case 32: SG_KN(launchStaged)<32>(pdl, g, stagedSmem, s, tab, rc, pos, acc, nn, nbl, rho, posF, Fv, fric, rowStride, eamTab); break;
+      default: SG_KN(launchStaged)<16>(pdl, g, stagedSmem, s, tab, rc, pos, acc, nn, nbl, rho, posF, Fv, fric, rowStride, eamTab);
     }
     return;
   }
@@ -473,23 +471,23 @@ void SG_KN(launchMetalChain)(bool pdl, int mt, int grid, int stagedGrid, size_t 
 #endif
   switch (mt) {
     case 4:
-      launchK(pdl, SG_KN(k_rho_tpa)<4>, grid, 128, 0, s, tab, rc, pos, nn, nbl, rho, dF, Fv, rowStride SG_EAM_ARG);
-      launchK(pdl, SG_KN(k_force_metal_tpa)<4>, grid, 128, 0, s, tab, rc, pos, acc, nn, nbl, dF, Fv, fric,
+      launchK(pdl, SG_KN(k_rho_tpa)<4>, grid, 128, 0, s, tab, rc, pos, nn, nbl, rho, posF, Fv, rowStride SG_EAM_ARG);
+      launchK(pdl, SG_KN(k_force_metal_tpa)<4>, grid, 128, 0, s, tab, rc, pos, acc, nn, nbl, posF, Fv, fric,
               rowStride SG_EAM_ARG);
       break;
     case 8:
-      launchK(pdl, SG_KN(k_rho_tpa)<8>, grid, 128, 0, s, tab, rc, pos, nn, nbl, rho, dF, Fv, rowStride SG_EAM_ARG);
-      launchK(pdl, SG_KN(k_force_metal_tpa)<8>, grid, 128, 0, s, tab, rc, pos, acc, nn, nbl, dF, Fv, fric,
+      launchK(pdl, SG_KN(k_rho_tpa)<8>, grid, 128, 0, s, tab, rc, pos, nn, nbl, rho, posF, Fv, rowStride SG_EAM_ARG);
+      launchK(pdl, SG_KN(k_force_metal_tpa)<8>, grid, 128, 0, s, tab, rc, pos, acc, nn, nbl, posF, Fv, fric,
               rowStride SG_EAM_ARG);
       break;
     case 32:
-      launchK(pdl, SG_KN(k_rho_tpa)<32>, grid, 128, 0, s, tab, rc, pos, nn, nbl, rho, dF, Fv, rowStride SG_EAM_ARG);
-      launchK(pdl, SG_KN(k_force_metal_tpa)<32>, grid, 128, 0, s, tab, rc, pos, acc, nn, nbl, dF, Fv, fric,
+      launchK(pdl, SG_KN(k_rho_tpa)<32>, grid, 128, 0, s, tab, rc, pos, nn, nbl, rho, posF, Fv, rowStride SG_EAM_ARG);
+      launchK(pdl, SG_KN(k_force_metal_tpa)<32>, grid, 128, 0, s, tab, rc, pos, acc, nn, nbl, posF, Fv, fric,
               rowStride SG_EAM_ARG);
       break;
     default:
-      launchK(pdl, SG_KN(k_rho), grid, 128, 0, s, tab, rc, pos, nn, nbl, rho, dF, Fv, rowStride SG_EAM_ARG);
-      launchK(pdl, SG_KN(k_force_metal), grid, 128, 0, s, tab, rc, pos, acc, nn, nbl, dF, Fv, fric,
+      launchK(pdl, SG_KN(k_rho), grid, 128, 0, s, tab, rc, pos, nn, nbl, rho, posF, Fv, rowStride SG_EAM_ARG);
+      launchK(pdl, SG_KN(k_force_metal), grid, 128, 0, s, tab, rc, pos, acc, nn, nbl, posF, Fv, fric,
               rowStride SG_EAM_ARG);
   }
 }

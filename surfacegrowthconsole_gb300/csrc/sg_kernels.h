@@ -34,17 +34,17 @@ __global__ void k_build_nebr_lanes(const int *tileRep, const int *active, const 
 
 // ---- PLAIN force and step kernels ----
 __global__ void k_rho(BlockTab tab, const RepConst *rc, const float4 *pos, const int *nn,
-                      const int *nbl, float *rho, float *dF, float *Fv, int rowStride);
+                      const int *nbl, float *rho, float4 *posF, float *Fv, int rowStride);
 __global__ void k_force_metal(BlockTab tab, const RepConst *rc, float4 *pos, float4 *acc,
-                              const int *nn, const int *nbl, const float *dF, const float *Fv,
+                              const int *nn, const int *nbl, const float4 *posF, const float *Fv,
                               float *fric, int rowStride);
 __global__ void k_force_both(BlockTab metal, BlockTab carbon, const RepConst *rc, float4 *pos, float4 *acc, const int *nn,
                              const int *nbl, const int *ns, const int *sl, const int *nrl, const unsigned *rl,
-                             const float *dF, const float *Fv, float *fric, int rowStride);
+                             const float4 *posF, const float *Fv, float *fric, int rowStride);
 // the metal chain (k_rho, k_force_metal) with mt lanes per atom (4, 8, 16, 32) on the table of
 // 128 / mt atoms per block
 void launchMetalChain(bool pdl, int mt, int grid, int stagedGrid, size_t stagedSmem, cudaStream_t s, BlockTab tab, const RepConst *rc, float4 *pos,
-                      float4 *acc, const int *nn, const int *nbl, float *rho, float *dF, float *Fv,
+                      float4 *acc, const int *nn, const int *nbl, float *rho, float4 *posF, float *Fv,
                       float *fric, int rowStride);
 // the carbon pass with minBlocks (8, 12, 16) resident 128-thread blocks per SM
 cudaError_t launchCarbon(bool pdl, int minBlocks, int grid, cudaStream_t s, BlockTab tab, const RepConst *rc,

@@ -21,6 +21,7 @@
 //    which puts 0 inside every min/max).
 #include <cuda_runtime.h>
 
+#include <cstring>
 #include <vector>
 
 #include "sg_device.cuh"
@@ -63,6 +64,8 @@ struct MixedBufs {
   int mixAtoms = kMixAtoms;     // atoms per step-reduction block (512, 1024, 2048 or 4096)
   int *redRep = nullptr, *redStart = nullptr;  // reduction blocks: replica, block index in it
   int redN = 0;
+  // start of each replica's own table; replicas whose tables are alike read the first one's (tabOff)
+  std::vector<int> ownTab;
   size_t stagedSmem = 0;        // shared memory of the staged metal kernels (the largest table)
   bool stagedOk = false;
 };
@@ -693,7 +696,8 @@ struct PersistArgs {
   int *nn, *nbl, *ns, *sl, *nrl;
   unsigned *rl;
   int rowStride, nebrMax, descending;
-  float *rho, *dF, *Fv, *fric;
+  float *rho, *Fv, *fric;
+  float4 *posF;
   const float4 *eamTab;
   float2 *partDF;
   float *partF;
@@ -767,7 +771,7 @@ __global__ void __launch_bounds__(128) k_step_persistent(PersistArgs a) {
   for (int e = blockIdx.x; e < nm + nc; e += G) {
     if (e < nm) {
       const RepConst &P = a.rc[a.metalTab.rep[e]];
-      rhoBody_mixed<MT>(e, P, a.metalTab, a.pos, a.nn, a.nbl, a.rho, a.dF, a.Fv, a.rowStride, a.eamTab + 2 * P.tabOff);
+      rhoBody_mixed<MT>(e, P, a.metalTab, a.pos, a.nn, a.nbl, a.rho, a.posF, a.Fv, a.rowStride, a.eamTab + 2 * P.tabOff);
     } else {
       carbonBody_mixed(e - nm, a.carbonTab, a.rc, a.pos, a.acc, a.nn, a.nbl, a.ns, a.sl, a.nrl, a.rl, a.rowStride);
     }
@@ -776,7 +780,7 @@ __global__ void __launch_bounds__(128) k_step_persistent(PersistArgs a) {
   if (!gridBarrier(a)) return;
   for (int e = blockIdx.x; e < nm; e += G) {
     const RepConst &P = a.rc[a.metalTab.rep[e]];
-    forceMetalBody_mixed<MT>(e, P, a.metalTab, a.pos, a.acc, a.nn, a.nbl, a.dF, a.Fv, a.fric, a.rowStride,
+    forceMetalBody_mixed<MT>(e, P, a.metalTab, a.pos, a.acc, a.nn, a.nbl, a.posF, a.Fv, a.fric, a.rowStride,
                              a.eamTab + 2 * P.tabOff);
   }
   if (!gridBarrier(a)) return;
@@ -850,6 +854,19 @@ int sg_mixed_init(sg_ctx *c) {
       eamPairExact(P, rmin + (k + 1) * h, b);
       for (int fn = 0; fn < 2; fn++) tab.push_back(hermite(a[2 * fn], a[2 * fn + 1], b[2 * fn], b[2 * fn + 1], h));
     }
+  }
+  // replicas of one metal share a table: 32 KB that stay in every L1 instead of 32 KB a replica
+  m->ownTab.resize(c->nrep);
+  int firstTab = -1;
+  for (int r = 0; r < c->nrep; r++) {
+    RepConst &P = c->hrc[r];
+    m->ownTab[r] = P.tabOff;
+    if (P.nTab == 0) continue;
+    if (firstTab < 0) firstTab = r;
+    const RepConst &F = c->hrc[firstTab];
+    if (P.nTab == F.nTab && P.rTabMin == F.rTabMin && P.rTabH == F.rTabH &&
+        memcmp(&tab[2 * (size_t)P.tabOff], &tab[2 * (size_t)m->ownTab[firstTab]], 2 * sizeof(float4) * P.nTab) == 0)
+      P.tabOff = m->ownTab[firstTab];
   }
   // the staged metal kernels hold the largest replica table in shared memory
   int maxTab = 0;
@@ -960,7 +977,7 @@ int sg_mixed_enqueue_forces(sg_ctx *c) {
     MCK(cudaStreamWaitEvent(c->side, c->evFork, 0));
     launchMetalChain_mixed(c->pdl, c->metalLanes, c->metalRun.n, c->eamStaged ? c->numSMs * 4 : 0,
                            m->stagedSmem, c->side, c->metalRun.view(), c->rc, c->pos, c->acc,
-                           c->nn, c->nbl, c->rho, c->dF, c->Fv, c->fric, c->rowStride, m->eamTab);
+                           c->nn, c->nbl, c->rho, c->posF, c->Fv, c->fric, c->rowStride, m->eamTab);
     if (c->opt.phase_timing) cudaEventRecordWithFlags(c->phaseEv[7], c->side, cudaEventRecordExternal);
     MCK(cudaGetLastError());
   }
@@ -1008,6 +1025,7 @@ extern "C" int sg_load_diff_theta(sg_ctx *c, int rep, const double *theta) {
     return sg_fail(SG_ERR_UNSUPPORTED, "sg_load_diff_theta: tables exist in MIXED mode only");
   MixedBufs *m = static_cast<MixedBufs *>(c->mixed);
   constexpr int kSC = SG_DIFF_SPLINE_COEFFS, kSI = SG_DIFF_SPLINE_INTERVALS;
+  for (int r = 0; r < c->nrep; r++) c->hrc[r].tabOff = m->ownTab[r];  // a table of its own again
   for (int r = (rep < 0 ? 0 : rep); r < (rep < 0 ? c->nrep : rep + 1); r++) {
     RepConst &P = c->hrc[r];
     if (P.nMolMe == 0) continue;
@@ -1073,7 +1091,7 @@ int sg_mixed_enqueue_persistent(sg_ctx *c, int forceRebuild) {
   a.sortIdx = c->sortIdx; a.sortPos = c->sortPos;
   a.nn = c->nn; a.nbl = c->nbl; a.ns = c->ns; a.sl = c->sl; a.nrl = c->nrl; a.rl = c->rl;
   a.rowStride = c->rowStride; a.nebrMax = c->nebrMax; a.descending = c->nebrDescending;
-  a.rho = c->rho; a.dF = c->dF; a.Fv = c->Fv; a.fric = c->fric;
+  a.rho = c->rho; a.posF = c->posF; a.Fv = c->Fv; a.fric = c->fric;
   a.eamTab = m->eamTab;
   a.partDF = m->partDF; a.partF = m->partF; a.redFirst = c->dRedFirst; a.counter = m->counter;
   a.diff64 = m->diff64; a.diffOff64 = m->dDiffOff64; a.diffF = c->diffBuf; a.diffOffF = c->dDiffOff;

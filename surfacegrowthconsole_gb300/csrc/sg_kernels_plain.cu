@@ -195,11 +195,11 @@ __global__ void __launch_bounds__(128, 8) k_force_both(BlockTab metal, BlockTab 
                                                        const int *__restrict__ nn, const int *__restrict__ nbl,
                                                        const int *__restrict__ ns, const int *__restrict__ sl,
                                                        const int *__restrict__ nrl, const unsigned *__restrict__ rl,
-                                                       const float *__restrict__ dF, const float *__restrict__ Fv,
+                                                       const float4 *__restrict__ posF, const float *__restrict__ Fv,
                                                        float *__restrict__ fric, int rowStride) {
   pdlEnter();
   if ((int)blockIdx.x < metal.nblocks)
-    forceMetalBody<kMT>(blockIdx.x, rc[metal.rep[blockIdx.x]], metal, pos, acc, nn, nbl, dF, Fv, fric, rowStride);
+    forceMetalBody<kMT>(blockIdx.x, rc[metal.rep[blockIdx.x]], metal, pos, acc, nn, nbl, posF, Fv, fric, rowStride);
   else
     carbonBody(blockIdx.x - metal.nblocks, carbon, rc, pos, acc, nn, nbl, ns, sl, nrl, rl, rowStride);
 }

@@ -47,7 +47,7 @@ static __device__ __align__(256) unsigned char g_scratch[kScratchBytes];
 // Carving of the scratch array (offsets in bytes, each 256-byte aligned).
 struct Carve {
   size_t rc, st, tabRep, tabStart, tileRep, cellStart;
-  size_t cellOf, sortIdx, nn, ns, sl, sortPos, rho, dF, Fv, fric, nbl, nrl, rl, active, heavy, work, total;
+  size_t cellOf, sortIdx, nn, ns, sl, sortPos, rho, posF, Fv, fric, nbl, nrl, rl, active, heavy, work, total;
 };
 constexpr size_t up(size_t x) { return (x + 255) & ~size_t(255); }
 constexpr Carve carve() {
@@ -67,7 +67,7 @@ constexpr Carve carve() {
   c.sl = o; o += up(N * kShortMax * sizeof(int));
   c.sortPos = o; o += up(N * sizeof(float4));
   c.rho = o; o += up(N * sizeof(float));
-  c.dF = o; o += up(N * sizeof(float));
+  c.posF = o; o += up(N * sizeof(float4));
   c.Fv = o; o += up(N * sizeof(float));
   c.fric = o; o += up(N * sizeof(float));
   c.nbl = o; o += up(N * SG_NOALLOC_MAX_NEBR * sizeof(int));
@@ -316,8 +316,9 @@ extern "C" int sg_compute_forces_noalloc(const sg_simparams *p, sg_float4 *d_pos
   int *cellOf = (int *)(base + K.cellOf), *sortIdx = (int *)(base + K.sortIdx), *nn = (int *)(base + K.nn), *ns = (int *)(base + K.ns);
   int *sl = (int *)(base + K.sl);
   float4 *sortPos = (float4 *)(base + K.sortPos);
-  float *rho = (float *)(base + K.rho), *dF = (float *)(base + K.dF), *Fv = (float *)(base + K.Fv);
+  float *rho = (float *)(base + K.rho), *Fv = (float *)(base + K.Fv);
   float *fric = (float *)(base + K.fric);
+  float4 *posF = (float4 *)(base + K.posF);
   int *nbl = (int *)(base + K.nbl), *nrl = (int *)(base + K.nrl);
   unsigned *rl = (unsigned *)(base + K.rl);
   int *active = (int *)(base + K.active), *work = (int *)(base + K.work);
@@ -340,8 +341,8 @@ extern "C" int sg_compute_forces_noalloc(const sg_simparams *p, sg_float4 *d_pos
   launchK(true, k_build_nebr, kBuildBlocks, kNebrWarps * 32, 0, s, tileRep, active, heavy, work, rc, st, cellStart, sortPos, nn,
           nbl, ns, sl, nrl, rl, rowStride, p->iNebrMax, 0, nullptr, 0);
   if (nMetalBlk)
-    launchK(true, k_rho, nMetalBlk, kBs, 0, s, metalTab, rc, pos, nn, nbl, rho, dF, Fv, rowStride);
-  launchK(true, k_force_both, nMetalBlk + nCarbBlk, kBs, 0, s, metalTab, carbTab, rc, pos, acc, nn, nbl, ns, sl, nrl, rl, dF, Fv,
+    launchK(true, k_rho, nMetalBlk, kBs, 0, s, metalTab, rc, pos, nn, nbl, rho, posF, Fv, rowStride);
+  launchK(true, k_force_both, nMetalBlk + nCarbBlk, kBs, 0, s, metalTab, carbTab, rc, pos, acc, nn, nbl, ns, sl, nrl, rl, posF, Fv,
           fric, rowStride);
   e = cudaGetLastError();
   if (e != cudaSuccess) return sg_fail(SG_ERR_CUDA, "sg_compute_forces_noalloc launch: %s", cudaGetErrorString(e));
