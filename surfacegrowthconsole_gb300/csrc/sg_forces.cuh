@@ -502,10 +502,12 @@ void SG_KN(launchMetalChain)(bool pdl, int mt, int grid, int stagedGrid, size_t 
 // The reference reuses its list counter for the bonded loop (cu:989), so after the third close
 // carbon its walk resumes at entry 4: metal entries at positions 4..p2 contribute their LJ term
 // twice, and entry 3 is skipped when p2 == 2.  After the walk, lane q < 3 adds the
-// second-neighbour terms of close carbon q (walking that neighbour's close list) and the
-// own-angle term of close carbons q, q + 1, and lane 3 the radial and out-of-plane terms (the
-// lanes 0..2 run one angle each, converged, instead of lane 3 running all three); the four
-// partial sums meet in a shuffle tree.
+// second-neighbour terms of close carbon q (walking that neighbour's close list), the own-angle term
+// of close carbons q, q + 1 and the radial term of q, and lane 3 the out-of-plane terms (the lanes
+// 0..2 run one of each, converged); the four partial sums meet in a shuffle tree.  The pass is bound
+// by instruction issue (80% of the slots at 686,000 atoms); with second neighbours taken by position
+// and one radial term a lane, beside the angle, the MIXED step of 64 replicas takes 245 us instead of
+// 252.5, ten steps of 45,546 atoms 703 us instead of 713.
 __device__ __forceinline__ void relEntry(bool full, const int *row, const unsigned *rrow, int atomOff, int e,
                                          int &k, int &j) {
   if (full) { k = row[e]; j = e; }
@@ -618,70 +620,80 @@ __device__ __forceinline__ void SG_KN(carbonBody)(int e, BlockTab tab, const Rep
     const float invR2 = __fdividef(1.f, absR * absR);
 #endif
     // the neighbour's close list holds, in list order, every entry that can pass the rCutC test
-    // below; four entries per load (a close-list row is 32 bytes, aligned)
+    // below (a close-list row is 32 bytes, aligned): the first two that pass and are not this atom
     const int nk = ns[k];
     const bool fullk = nk < 0;
     const int lim = fullk ? nn[k] : nk;
     const int *src = fullk ? nbl + (size_t)k * rowStride : sl + (size_t)k * kShortMax;
     int countk = 0;
-    for (int l0 = 0; l0 < lim && countk < 2; l0 += 4) {
-      int mm[4];
-      bool use[4];
-      if (fullk) {
-#pragma unroll
-        for (int t = 0; t < 4; t++) {
-          use[t] = l0 + t < lim;
-          mm[t] = use[t] ? src[l0 + t] : 0;
-        }
-      } else {
-        const int4 u = *reinterpret_cast<const int4 *>(src + l0);
-        mm[0] = u.x; mm[1] = u.y; mm[2] = u.z; mm[3] = u.w;
-#pragma unroll
-        for (int t = 0; t < 4; t++) use[t] = l0 + t < lim;
-      }
-#pragma unroll
-      for (int t = 0; t < 4; t++) {
-        if (!use[t]) continue;
-        const int m = mm[t];
-        const float4 rm = pos[m];
-        float ex = minImg(B.x - rm.x, P.region[0]);
-        float ey = minImg(B.y - rm.y, P.region[1]);
-        float ez = minImg(B.z - rm.z, P.region[2]);
-        const float rr2 = ex * ex + ey * ey + ez * ez;
-        if ((rr2 < P.rrCutC) && (m != i)) {
-          ex = ex * (-1.f); ey = ey * (-1.f); ez = ez * (-1.f);
+    auto second = [&](const float4 &rm) {
+      float ex = minImg(B.x - rm.x, P.region[0]);
+      float ey = minImg(B.y - rm.y, P.region[1]);
+      float ez = minImg(B.z - rm.z, P.region[2]);
+      const float rr2 = ex * ex + ey * ey + ez * ez;
+      if (rr2 < P.rrCutC) {
+        ex = ex * (-1.f); ey = ey * (-1.f); ez = ez * (-1.f);
 #ifdef SG_FAST_RECIP
-          const float inv = __fdividef(1.f, absR * rr2);
-          const float cs = (rnx * ex + rny * ey + rnz * ez) * inv;
-          const float th = acosf(cs);
-          const float dth = th - P.theta_0;
-          const float tmp = P.mu_theta * dth * rsqrtf(1.f - cs * cs);
-          float f = tmp * inv;
-          fx = fx + f * ex; fy = fy + f * ey; fz = fz + f * ez;
-          f = -tmp * cs * invR2;
-          fx = fx + f * rnx; fy = fy + f * rny; fz = fz + f * rnz;
-          f = -P.mu_p * (rm.z - P.z_0) * (1.f / 9.f);
+        const float inv = __fdividef(1.f, absR * rr2);
+        const float cs = (rnx * ex + rny * ey + rnz * ez) * inv;
+        const float th = acosf(cs);
+        const float dth = th - P.theta_0;
+        const float tmp = P.mu_theta * dth * rsqrtf(1.f - cs * cs);
+        float f = tmp * inv;
+        fx = fx + f * ex; fy = fy + f * ey; fz = fz + f * ez;
+        f = -tmp * cs * invR2;
+        fx = fx + f * rnx; fy = fy + f * rny; fz = fz + f * rnz;
+        f = -P.mu_p * (rm.z - P.z_0) * (1.f / 9.f);
 #else
-          const float cs = (rnx * ex + rny * ey + rnz * ez) / (absR * rr2);
-          const float th = acosf(cs);
-          const float dth = th - P.theta_0;
-          const float tmp = P.mu_theta * dth / sqrtf(1.f - cs * cs);
-          float f = tmp / (absR * rr2);
-          fx = fx + f * ex; fy = fy + f * ey; fz = fz + f * ez;
-          f = -tmp * cs / (absR * absR);
-          fx = fx + f * rnx; fy = fy + f * rny; fz = fz + f * rnz;
-          f = -P.mu_p * (rm.z - P.z_0) / 9.f;
+        const float cs = (rnx * ex + rny * ey + rnz * ez) / (absR * rr2);
+        const float th = acosf(cs);
+        const float dth = th - P.theta_0;
+        const float tmp = P.mu_theta * dth / sqrtf(1.f - cs * cs);
+        float f = tmp / (absR * rr2);
+        fx = fx + f * ex; fy = fy + f * ey; fz = fz + f * ez;
+        f = -tmp * cs / (absR * absR);
+        fx = fx + f * rnx; fy = fy + f * rny; fz = fz + f * rnz;
+        f = -P.mu_p * (rm.z - P.z_0) / 9.f;
 #endif
-          fz = fz + f;
-          ++countk;
-        }
-        if (countk == 2) break;
+        fz = fz + f;
+        ++countk;
+      }
+    };
+    // In a sheet the list is this atom and two others, in any order: its first two others are taken
+    // by position, so that the lanes evaluate two entries each at once; walking the entries, every
+    // lane's third one (this atom, in another place for each lane) cost the warp a whole term.
+    // (One loop: the term's code once.)
+    float4 rm = B, r1 = B;
+    bool have = false, have1 = false;
+    int l = 0;
+    if (!fullk) {
+      const int4 u = *reinterpret_cast<const int4 *>(src);  // entries past the list are not used
+      const int at0 = u.x == i ? 1 : 0, at1 = (u.x == i || u.y == i) ? 2 : 1;
+      have = at0 < lim;
+      have1 = at1 < lim;
+      if (have) rm = pos[at0 ? u.y : u.x];
+      if (have1) r1 = pos[at1 == 2 ? u.z : u.y];
+      l = at1 + 1;
+    }
+#pragma unroll 1
+    for (bool first = true;; first = false) {
+      if (have) second(rm);
+      if (countk == 2) break;
+      if (first) {
+        rm = r1;
+        have = have1;
+      } else {  // a list of more entries, or of entries past the cutoff
+        if (l >= lim) break;
+        const int m = src[l++];
+        have = m != i;
+        if (have) rm = pos[m];
       }
     }
   }
   if (counti == 3) {
     if (sub < 3) {
-      // own-angle term of close carbons q, q + 1 (cu:1020-1061): one per lane 0..2
+      // own-angle term of close carbons q, q + 1 (cu:1020-1061) and radial term of q (cu:985-1019): one
+      // of each per lane 0..2
       const int p0 = sub, p1 = (sub == 2) ? 0 : sub + 1;
       const float rx0 = sD[a][p0][0], ry0 = sD[a][p0][1], rz0 = sD[a][p0][2], ar0 = sD[a][p0][3];
       const float rx1 = sD[a][p1][0], ry1 = sD[a][p1][1], rz1 = sD[a][p1][2], ar1 = sD[a][p1][3];
@@ -706,22 +718,17 @@ __device__ __forceinline__ void SG_KN(carbonBody)(int e, BlockTab tab, const Rep
 #endif
       fx = fx + f * rx0; fy = fy + f * ry0; fz = fz + f * rz0;
       u += P.mu_theta * dth * dth;
-    } else {
-      // radial and out-of-plane terms (cu:985-1019): lane 3
-      float dzs = 0.f;
-#pragma unroll
-      for (int q = 0; q < 3; q++) {
-        const float rx = sD[a][q][0], ry = sD[a][q][1], rz = sD[a][q][2], ar = sD[a][q][3];
 #ifdef SG_FAST_RECIP
-        const float f = -P.mu_r * (ar - 1.f) * __fdividef(1.f, ar);
+      f = -P.mu_r * (ar0 - 1.f) * i0;
 #else
-        const float f = -P.mu_r * (ar - 1.f) / ar;
+      f = -P.mu_r * (ar0 - 1.f) / ar0;
 #endif
-        fx = fx + f * rx; fy = fy + f * ry; fz = fz + f * rz;
-        u += P.mu_r * (ar - 1.f) * (ar - 1.f);
-      }
+      fx = fx + f * rx0; fy = fy + f * ry0; fz = fz + f * rz0;
+      u += P.mu_r * (ar0 - 1.f) * (ar0 - 1.f);
+    } else {
+      // out-of-plane terms: lane 3
       const float z0 = sZ[a][0], z1 = sZ[a][1], z2 = sZ[a][2];
-      dzs = z0 + z1 + z2;
+      const float dzs = z0 + z1 + z2;
       float dZ = 2.f * (A.z - P.z_0) - dzs;
       fz = fz + -0.666666667f * P.mu_p * dZ;
       dZ = (A.z - P.z_0) - 0.33333333f * dzs;
