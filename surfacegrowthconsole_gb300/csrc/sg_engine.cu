@@ -87,16 +87,25 @@ static int uploadTab(sg_ctx *c, DevTab &t, const std::vector<int> &rep, const st
   }
   return SG_OK;
 }
-// blocks of bs over [b, e) of each replica
-static int makeRangeTab(sg_ctx *c, DevTab &t, int bs, int which) {
-  std::vector<int> rep, start;
+// blocks of bs over the atoms (which 0), metal atoms (1) or carbon atoms (2) of each replica
+int sg_make_range_tab(sg_ctx *c, DevTab &t, int bs, int which) {
+  std::vector<int> rep, start, stop;
   for (int r = 0; r < c->nrep; r++) {
     const RepConst &P = c->hrc[r];
     int b = P.atomOff, e = P.atomOff + P.nMol;
     if (which == 1) e = P.atomOff + P.nMolMe;
     if (which == 2) b = P.atomOff + P.nMolMe;
-    for (int s = b; s < e; s += bs) { rep.push_back(r); start.push_back(s); }
+    for (int s = b; s < e; s += bs) { rep.push_back(r); start.push_back(s); stop.push_back(e); }
+    if (c->nrep == 1) {
+      t.first = b;
+      t.step = bs;
+      t.end = e;
+    }
   }
+  int rc;
+  if ((rc = devAllocT(c, &t.stop, std::max<size_t>(stop.size(), 1)))) return rc;
+  if (!stop.empty())
+    CK(cudaMemcpyAsync(t.stop, stop.data(), stop.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
   return uploadTab(c, t, rep, start);
 }
 
@@ -185,7 +194,7 @@ static int setMetalLanes(sg_ctx *c, int lanes) {
     return sg_fail(SG_ERR_UNSUPPORTED, "metal_lanes %d: the persistent step runs 4 or %d", lanes, kMT);
   DevTab &t = c->metalLaneTab[slot];
   if (!t.rep) {
-    const int rc = makeRangeTab(c, t, 128 / lanes, 1);
+    const int rc = sg_make_range_tab(c, t, 128 / lanes, 1);
     if (rc) return rc;
   }
   if (lanes != c->metalLanes) destroyGraphs(c);
@@ -399,9 +408,9 @@ extern "C" int sg_create(const sg_simparams *params, int n_replicas, const sg_op
   if (c->opt.phase_timing)
     for (auto &e : c->phaseEv) cudaEventCreate(&e);
   // tables
-  if ((rc = makeRangeTab(c, c->atomTab, 128, 0)) || (rc = makeRangeTab(c, c->metalTab, 128, 1)) ||
-      (rc = makeRangeTab(c, c->carbonTab, 128, 2)) || (rc = makeRangeTab(c, c->metalTabT, kMetalPerBlock, 1)) ||
-      (rc = makeRangeTab(c, c->carbonTabT, kCarbonPerBlock, 2)) || (rc = makeRangeTab(c, c->rdfTab, kRdfAtoms, 1))) {
+  if ((rc = sg_make_range_tab(c, c->atomTab, 128, 0)) || (rc = sg_make_range_tab(c, c->metalTab, 128, 1)) ||
+      (rc = sg_make_range_tab(c, c->carbonTab, 128, 2)) || (rc = sg_make_range_tab(c, c->metalTabT, kMetalPerBlock, 1)) ||
+      (rc = sg_make_range_tab(c, c->carbonTabT, kCarbonPerBlock, 2)) || (rc = sg_make_range_tab(c, c->rdfTab, kRdfAtoms, 1))) {
     sg_destroy(c);
     return rc;
   }
@@ -449,11 +458,9 @@ extern "C" int sg_create(const sg_simparams *params, int n_replicas, const sg_op
     }
   }
   {
-    std::vector<int> rr, ss, cr, cs, tr, ts;
+    std::vector<int> tr, ts;
     for (int r = 0; r < n_replicas; r++) {
       const RepConst &P = c->hrc[r];
-      for (int b = 0; b < P.nRedBlocks; b++) { rr.push_back(r); ss.push_back(b); }
-      for (int b = 0; b < (P.nMolMe + kRedElems - 1) / kRedElems; b++) { cr.push_back(r); cs.push_back(b); }
       c->tileFirst.push_back((int)tr.size());
       for (int t = 0; t < P.ncellsPad; t += kCellTile) { tr.push_back(r); ts.push_back(t); }
     }
@@ -464,7 +471,7 @@ extern "C" int sg_create(const sg_simparams *params, int n_replicas, const sg_op
                        ? 2 * kScanCells : kScanCells;
     for (auto &P : c->hrc) P.scanCells = c->scanCells;
     c->nScanBlocks = c->ntiles * (kCellTile / c->scanCells);
-    if ((rc = uploadTab(c, c->redTab, rr, ss)) || (rc = uploadTab(c, c->cmvTab, cr, cs)) ||
+    if ((rc = sg_make_range_tab(c, c->redTab, kRedElems, 0)) || (rc = sg_make_range_tab(c, c->cmvTab, kRedElems, 1)) ||
         (rc = uploadTab(c, c->tileTab, tr, ts))) {
       sg_destroy(c);
       return rc;
@@ -714,7 +721,7 @@ enum { V_SHEAR = 1, V_RDF = 2, V_RDF_ZERO = 4, G_FROM_HOST = 256, G_PUBLISH = 51
 
 static int enqueueRebuild(sg_ctx *c, int force) {
   const int fr = force;
-  CK(launchScanRank(c->pdl, c->scanCells, c->nScanBlocks, c->stream, c->tileTab.rep, c->tileTab.start,
+  CK(launchScanRank(c->pdl, c->scanCells, c->nScanBlocks, c->stream, c->tileReps(), c->tileTab.start,
              c->dTileFirst, c->rc, c->st, c->cellCount, c->cellStart, c->bucketCap, fr, c->activeCells,
              c->heavyItems, c->nebrWork, c->nebrItemAtoms, c->blockCount, c->bucket, c->spill, c->cellOf, c->pos,
              c->sortIdx, c->sortPos, c->nn, c->ns, c->nrl));
@@ -725,7 +732,7 @@ static int enqueueRebuild(sg_ctx *c, int force) {
                c->nebrMax, c->nebrWork, fr, c->blockCount, c->nScanBlocks));
   else
     CK(launchK(c->pdl, c->nebrAlgo == 2 ? k_build_nebr_lanes : k_build_nebr, c->nebrGrid, kNebrWarps * 32, 0,
-               c->stream, c->tileTab.rep, c->activeCells,
+               c->stream, c->tileReps(), c->activeCells,
                c->heavyItems, c->nebrWork, c->rc, c->st, c->cellStart, c->sortPos, c->nn, c->nbl, c->ns, c->sl,
                c->nrl, c->rl, c->rowStride, c->nebrMax, c->nebrDescending, c->blockCount, c->nScanBlocks));
   return SG_OK;

@@ -16,9 +16,10 @@ using sg::RepState;
 
 // ---- host-side tables ----------------------------------------------------------------------
 struct DevTab {
-  int *rep = nullptr, *start = nullptr;
+  int *rep = nullptr, *start = nullptr, *stop = nullptr;
   int n = 0;
-  BlockTab view() const { return BlockTab{rep, start, n}; }
+  int first = 0, step = 0, end = 0;  // of one replica: the entries as a sequence
+  BlockTab view() const { return BlockTab{rep, start, n, stop, first, step, end}; }
 };
 
 // The host buffers a step-from-host graph reads (replica, r, v, a).
@@ -68,6 +69,8 @@ struct sg_ctx {
   float *diffBuf = nullptr;
   size_t *dDiffOff = nullptr;
   DevTab atomTab, metalTab, carbonTab, redTab, cmvTab, tileTab;
+  // the cell tiles' replicas; none to look up with one replica
+  const int *tileReps() const { return nrep == 1 ? nullptr : tileTab.rep; }
   DevTab metalTabT, carbonTabT;  // blocks of kMetalPerBlock / kCarbonPerBlock atoms
   DevTab rdfTab;                 // blocks of kRdfAtoms metal atoms (the RDF sample)
   // launch shape of the metal chain: lanes per atom and its block table (128 / lanes atoms per
@@ -118,6 +121,7 @@ struct sg_ctx {
 int sg_fail(int code, const char *fmt, ...);
 
 void sg_populate(void *p, size_t bytes);
+int sg_make_range_tab(sg_ctx *c, DevTab &t, int bs, int which);
 int sg_read_state(sg_ctx *c, int rep, sg::RepState *out);
 int sg_get_diffusion_print(sg_ctx *c, int rep, float *table, int *nprints);
 int sg_next_variant(sg_ctx *c);

@@ -208,9 +208,9 @@ __device__ __forceinline__ void SG_KN(rhoBody)(int e, const RepConst &P, BlockTa
                                                int rowStride SG_EAM_BODY_PARAM) {
   const int sub = threadIdx.x & (MT - 1);
   const unsigned gmask = laneGroupMask<MT>();
-  const int i = tab.start[e] + threadIdx.x / MT;
+  const int i = tabStart(tab, e) + threadIdx.x / MT;
   const int metalEnd = P.atomOff + P.nMolMe;
-  const bool valid = i < metalEnd;
+  const bool valid = i < tabStop(tab, e);
   float sum = 0.f;
   float4 A = make_float4(0.f, 0.f, 0.f, 0.f);
   if (valid) {
@@ -219,11 +219,14 @@ __device__ __forceinline__ void SG_KN(rhoBody)(int e, const RepConst &P, BlockTa
     const int *row = nbl + (size_t)i * rowStride;
     // kMetalBatch entries per lane per round: their indices, then their positions, load
     // together; their densities are added in pairs (fewer roundings in sequence)
+    int k[kMetalBatch];  // the first round's indices leave before n is known
+#pragma unroll
+    for (int q = 0; q < kMetalBatch; q++) k[q] = (sub + q * MT < rowStride) ? row[sub + q * MT] : -1;
     for (int j0 = sub; j0 < n; j0 += kMetalBatch * MT) {
-      int k[kMetalBatch];
       float4 B[kMetalBatch];
 #pragma unroll
-      for (int q = 0; q < kMetalBatch; q++) k[q] = (j0 + q * MT < n) ? row[j0 + q * MT] : -1;
+      for (int q = 0; q < kMetalBatch; q++)
+        if (j0 + q * MT >= n) k[q] = -1;
 #pragma unroll
       for (int q = 0; q < kMetalBatch; q++) B[q] = (k[q] >= 0) ? pos[k[q]] : A;
       float d[kMetalBatch] = {};
@@ -241,6 +244,11 @@ __device__ __forceinline__ void SG_KN(rhoBody)(int e, const RepConst &P, BlockTa
 #endif
       }
       sum += (d[0] + d[1]) + (d[2] + d[3]);
+#pragma unroll
+      for (int q = 0; q < kMetalBatch; q++) {
+        const int j = j0 + (kMetalBatch + q) * MT;
+        if (j < n) k[q] = row[j];
+      }
     }
   }
 #pragma unroll
@@ -258,7 +266,7 @@ __global__ void __launch_bounds__(128) SG_KN(k_rho)(BlockTab tab, const RepConst
                                              float4 *__restrict__ posF, float *__restrict__ Fv,
                                              int rowStride SG_EAM_PARAM) {
   pdlEnter();
-  const RepConst &P = rc[tab.rep[blockIdx.x]];
+  const RepConst &P = rc[tabRep(tab, blockIdx.x)];
   SG_KN(rhoBody)<kMT>(blockIdx.x, P, tab, pos, nn, nbl, rho, posF, Fv, rowStride SG_EAM_BASE(P));
 }
 template <int MT>
@@ -268,7 +276,7 @@ __global__ void __launch_bounds__(128) SG_KN(k_rho_tpa)(BlockTab tab, const RepC
                                                  float4 *__restrict__ posF, float *__restrict__ Fv,
                                                  int rowStride SG_EAM_PARAM) {
   pdlEnter();
-  const RepConst &P = rc[tab.rep[blockIdx.x]];
+  const RepConst &P = rc[tabRep(tab, blockIdx.x)];
   SG_KN(rhoBody)<MT>(blockIdx.x, P, tab, pos, nn, nbl, rho, posF, Fv, rowStride SG_EAM_BASE(P));
 }
 
@@ -299,9 +307,9 @@ __device__ __forceinline__ void SG_KN(forceMetalBody)(int e, const RepConst &P, 
                                                       int rowStride SG_EAM_BODY_PARAM) {
   const int sub = threadIdx.x & (MT - 1);
   const unsigned gmask = laneGroupMask<MT>();
-  const int i = tab.start[e] + threadIdx.x / MT;
+  const int i = tabStart(tab, e) + threadIdx.x / MT;
   const int metalEnd = P.atomOff + P.nMolMe;
-  const bool valid = i < metalEnd;
+  const bool valid = i < tabStop(tab, e);
   float fx = 0.f, fy = 0.f, fz = 0.f, rx = 0.f, u = 0.f;
   if (valid) {
     const float4 A = posF[i];
@@ -309,11 +317,14 @@ __device__ __forceinline__ void SG_KN(forceMetalBody)(int e, const RepConst &P, 
     const float dFi = A.w;
     const int *row = nbl + (size_t)i * rowStride;
     // batches of entries as in the density pass; same order of the sums
+    int k[kMetalBatch];  // the first round's indices leave before n is known
+#pragma unroll
+    for (int q = 0; q < kMetalBatch; q++) k[q] = (sub + q * MT < rowStride) ? row[sub + q * MT] : -1;
     for (int j0 = sub; j0 < n; j0 += kMetalBatch * MT) {
-      int k[kMetalBatch];
       float4 B[kMetalBatch];
 #pragma unroll
-      for (int q = 0; q < kMetalBatch; q++) k[q] = (j0 + q * MT < n) ? row[j0 + q * MT] : -1;
+      for (int q = 0; q < kMetalBatch; q++)
+        if (j0 + q * MT >= n) k[q] = -1;
 #pragma unroll
       for (int q = 0; q < kMetalBatch; q++) B[q] = (k[q] >= 0) ? (k[q] < metalEnd ? posF : pos)[k[q]] : A;
 #pragma unroll
@@ -350,6 +361,11 @@ __device__ __forceinline__ void SG_KN(forceMetalBody)(int e, const RepConst &P, 
           rx = rx + fc * dx;
         }
       }
+#pragma unroll
+      for (int q = 0; q < kMetalBatch; q++) {
+        const int j = j0 + (kMetalBatch + q) * MT;
+        if (j < n) k[q] = row[j];
+      }
     }
   }
 #pragma unroll
@@ -373,7 +389,7 @@ __global__ void __launch_bounds__(128) SG_KN(k_force_metal)(BlockTab tab, const 
                                                      const float4 *__restrict__ posF, const float *__restrict__ Fv,
                                                      float *__restrict__ fric, int rowStride SG_EAM_PARAM) {
   pdlEnter();
-  const RepConst &P = rc[tab.rep[blockIdx.x]];
+  const RepConst &P = rc[tabRep(tab, blockIdx.x)];
   SG_KN(forceMetalBody)<kMT>(blockIdx.x, P, tab, pos, acc, nn, nbl, posF, Fv, fric, rowStride SG_EAM_BASE(P));
 }
 template <int MT>
@@ -384,7 +400,7 @@ __global__ void __launch_bounds__(128) SG_KN(k_force_metal_tpa)(BlockTab tab, co
                                                          const float *__restrict__ Fv, float *__restrict__ fric,
                                                          int rowStride SG_EAM_PARAM) {
   pdlEnter();
-  const RepConst &P = rc[tab.rep[blockIdx.x]];
+  const RepConst &P = rc[tabRep(tab, blockIdx.x)];
   SG_KN(forceMetalBody)<MT>(blockIdx.x, P, tab, pos, acc, nn, nbl, posF, Fv, fric, rowStride SG_EAM_BASE(P));
 }
 
@@ -402,7 +418,7 @@ __global__ void __launch_bounds__(128) SG_KN(k_rho_staged)(BlockTab tab, const R
   pdlEnter();
   int staged = -1;
   for (int e = blockIdx.x; e < tab.nblocks; e += gridDim.x) {
-    const int rep = tab.rep[e];
+    const int rep = tabRep(tab, e);
     const RepConst &P = rc[rep];
     if (rep != staged) {
       __syncthreads();
@@ -424,7 +440,7 @@ __global__ void __launch_bounds__(128) SG_KN(k_force_metal_staged)(BlockTab tab,
   pdlEnter();
   int staged = -1;
   for (int e = blockIdx.x; e < tab.nblocks; e += gridDim.x) {
-    const int rep = tab.rep[e];
+    const int rep = tabRep(tab, e);
     const RepConst &P = rc[rep];
     if (rep != staged) {
       __syncthreads();
@@ -527,15 +543,15 @@ __device__ __forceinline__ void SG_KN(carbonBody)(int e, BlockTab tab, const Rep
   __shared__ float sD[128 / kCT][3][4];  // dx, dy, dz, |d| of close carbon q
   __shared__ float sZ[128 / kCT][3];     // its z - z_0
   __shared__ int sK[128 / kCT][3];       // its index
-  const int rep = tab.rep[e];
+  const int rep = tabRep(tab, e);
   const RepConst &P = rc[rep];
   const int sub = threadIdx.x & (kCT - 1);
   const int a = threadIdx.x / kCT;  // atom slot in the block
   const int glane = threadIdx.x & 31 & ~(kCT - 1);
   const unsigned gmask = ((1u << kCT) - 1) << glane;
-  const int i = tab.start[e] + a;
+  const int i = tabStart(tab, e) + a;
   const int metalEnd = P.atomOff + P.nMolMe;
-  const bool valid = i < P.atomOff + P.nMol;
+  const bool valid = i < tabStop(tab, e);
   float fx = 0.f, fy = 0.f, fz = 0.f, u = 0.f;
   int counti = 0, p2 = -1;
   const float4 A = valid ? pos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -544,6 +560,7 @@ __device__ __forceinline__ void SG_KN(carbonBody)(int e, BlockTab tab, const Rep
   const int nEnt = full ? nn[i] : nr;
   const int *row = nbl + (size_t)i * rowStride;
   const unsigned *rrow = rl + (size_t)i * kRelMax;
+  const unsigned r0 = valid ? rrow[sub] : 0u;  // leaves before nr is known
   for (int base = 0; base < nEnt; base += kCT) {
     const int e = base + sub;
     bool closeC = false;
@@ -551,7 +568,8 @@ __device__ __forceinline__ void SG_KN(carbonBody)(int e, BlockTab tab, const Rep
     float dx = 0.f, dy = 0.f, dz = 0.f, rr = 0.f, bz = 0.f;
     int k = -1, j = -1;
     if (e < nEnt) {
-      relEntry(full, row, rrow, P.atomOff, e, k, j);
+      if (full || base > 0) relEntry(full, row, rrow, P.atomOff, e, k, j);
+      else relEntry(false, row, &r0, P.atomOff, 0, k, j);
       const float4 B = pos[k];
       bz = B.z;
       dx = minImg(A.x - B.x, P.region[0]);

@@ -62,8 +62,7 @@ struct MixedBufs {
   unsigned *counter = nullptr;  // per replica: blocks done
   float4 *eamTab = nullptr;     // per replica nTab intervals x 2: cubic coefficients of phi, of f
   int mixAtoms = kMixAtoms;     // atoms per step-reduction block (512, 1024, 2048 or 4096)
-  int *redRep = nullptr, *redStart = nullptr;  // reduction blocks: replica, block index in it
-  int redN = 0;
+  DevTab redTab;  // reduction blocks
   // start of each replica's own table; replicas whose tables are alike read the first one's (tabOff)
   std::vector<int> ownTab;
   size_t stagedSmem = 0;        // shared memory of the staged metal kernels (the largest table)
@@ -126,16 +125,15 @@ __device__ __forceinline__ void integrateMixedBody(int e, BlockTab tab, const Re
                                                    const float4 *__restrict__ hostR = nullptr,
                                                    const float *__restrict__ hostV = nullptr,
                                                    const float *__restrict__ hostA = nullptr) {
-  const int rep = tab.rep[e];
+  const int rep = tabRep(tab, e);
   const RepConst &P = rc[rep];
   RepState *S = st + rep;
-  const int g = tab.start[e] + threadIdx.x;
-  const int gEnd = P.atomOff + P.nMol;
+  const int g0 = tabStart(tab, e), g = g0 + threadIdx.x, gEnd = tabStop(tab, e);
   float4 r, lo, v, a;
   bool pending;
   if (hostR) {
     __shared__ float sV[3 * 128], sA[3 * 128];
-    const int g0 = tab.start[e], g1 = min(gEnd, g0 + (int)blockDim.x);
+    const int g1 = min(gEnd, g0 + (int)blockDim.x);
     if (g < gEnd) r = hostR[g];  // every read over the host link before the barrier
     stageRows3Range(hostV, g0, g1, sV);
     stageRows3Range(hostA, g0, g1, sA);
@@ -262,10 +260,10 @@ __device__ __forceinline__ void reduceMixedBody(
     const int *__restrict__ redFirst, unsigned *counter, double *__restrict__ diff64,
     const size_t *__restrict__ diffOff64, float *__restrict__ diffF, const size_t *__restrict__ diffOffF,
     int forceRebuild, const PublishArgs pub = PublishArgs{}) {
-  const int rep = tab.rep[e];
+  const int rep = tabRep(tab, e);
   const RepConst &P = rc[rep];
   RepState *S = st + rep;
-  const int b = tab.start[e];
+  const int g0 = tabStart(tab, e), stop = tabStop(tab, e);
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
   const float h = 0.5f * P.deltaT;
   // per thread and per warp (64 atoms) in FP32, except the centre of mass (double-float over
@@ -275,12 +273,10 @@ __device__ __forceinline__ void reduceMixedBody(
   for (int k = 0; k < kMixAcc; k++) acc[k] = 0.f;
   DF cm[3] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
   float mm[kMixMax] = {0.f, 3.4e38f, 3.4e38f, 3.4e38f, -3.4e38f, -3.4e38f, -3.4e38f};
-  const int atomsPerThread = APT > 0 ? APT : apt;
 #pragma unroll
   for (int half = 0; half < (APT > 0 ? APT : apt); half++) {
-    const int local = atomsPerThread * THREADS * b + half * THREADS + t;
-    if (local >= P.nMol) continue;
-    const int g = P.atomOff + local;
+    const int g = g0 + half * THREADS + t, local = g - P.atomOff;
+    if (g >= stop) continue;
     const float4 r = pos[g];
     float4 v = vel[g];
     const float4 a = acc4[g];
@@ -353,7 +349,7 @@ __device__ __forceinline__ void reduceMixedBody(
     if (lane == 0) shF[w][k] = x;
   }
   __syncthreads();
-  const int pb = P.redFirstM + b;
+  const int pb = e;  // the blocks' slots are in the order of the table
   if (t < kMixAcc) {
     DF x{0.f, 0.f};
     for (int k = 0; k < THREADS / 32; k++) x = dfAdd(x, shDF[k][t]);
@@ -770,7 +766,7 @@ __global__ void __launch_bounds__(128) k_step_persistent(PersistArgs a) {
   const int nm = a.metalTab.nblocks, nc = a.carbonTab.nblocks;
   for (int e = blockIdx.x; e < nm + nc; e += G) {
     if (e < nm) {
-      const RepConst &P = a.rc[a.metalTab.rep[e]];
+      const RepConst &P = a.rc[tabRep(a.metalTab, e)];
       rhoBody_mixed<MT>(e, P, a.metalTab, a.pos, a.nn, a.nbl, a.rho, a.posF, a.Fv, a.rowStride, a.eamTab + 2 * P.tabOff);
     } else {
       carbonBody_mixed(e - nm, a.carbonTab, a.rc, a.pos, a.acc, a.nn, a.nbl, a.ns, a.sl, a.nrl, a.rl, a.rowStride);
@@ -779,7 +775,7 @@ __global__ void __launch_bounds__(128) k_step_persistent(PersistArgs a) {
   }
   if (!gridBarrier(a)) return;
   for (int e = blockIdx.x; e < nm; e += G) {
-    const RepConst &P = a.rc[a.metalTab.rep[e]];
+    const RepConst &P = a.rc[tabRep(a.metalTab, e)];
     forceMetalBody_mixed<MT>(e, P, a.metalTab, a.pos, a.acc, a.nn, a.nbl, a.posF, a.Fv, a.fric, a.rowStride,
                              a.eamTab + 2 * P.tabOff);
   }
@@ -897,24 +893,19 @@ int sg_mixed_init(sg_ctx *c) {
         break;
       }
     }
-    std::vector<int> rr, ss;
+    int first = 0;
     for (int r = 0; r < c->nrep; r++) {
       RepConst &P = c->hrc[r];
       P.nRedBlocksM = (P.nMol + m->mixAtoms - 1) / m->mixAtoms;
-      P.redFirstM = (int)rr.size();
-      for (int b = 0; b < P.nRedBlocksM; b++) { rr.push_back(r); ss.push_back(b); }
+      P.redFirstM = first;
+      first += P.nRedBlocksM;
     }
-    m->redN = (int)rr.size();
-    MCK(cudaMalloc(&m->redRep, sizeof(int) * std::max<size_t>(rr.size(), 1)));
-    sg_register_region(c, m->redRep, sizeof(int) * std::max<size_t>(rr.size(), 1));
-    MCK(cudaMalloc(&m->redStart, sizeof(int) * std::max<size_t>(ss.size(), 1)));
-    sg_register_region(c, m->redStart, sizeof(int) * std::max<size_t>(ss.size(), 1));
-    MCK(cudaMemcpyAsync(m->redRep, rr.data(), sizeof(int) * rr.size(), cudaMemcpyHostToDevice, c->stream));
-    MCK(cudaMemcpyAsync(m->redStart, ss.data(), sizeof(int) * ss.size(), cudaMemcpyHostToDevice, c->stream));
+    const int rc = sg_make_range_tab(c, m->redTab, m->mixAtoms, 0);
+    if (rc) return rc;
     MCK(cudaMemcpyAsync(c->rc, c->hrc.data(), sizeof(RepConst) * c->nrep, cudaMemcpyHostToDevice, c->stream));
     MCK(cudaStreamSynchronize(c->stream));
   }
-  const int nRed = std::max(m->redN, 1);
+  const int nRed = std::max(m->redTab.n, 1);
   MCK(cudaMalloc(&m->partDF, sizeof(float2) * nRed * kMixAcc));
   sg_register_region(c, m->partDF, sizeof(float2) * nRed * kMixAcc);
   MCK(cudaMalloc(&m->partF, sizeof(float) * nRed * kMixMax));
@@ -949,8 +940,6 @@ void sg_mixed_free(sg_ctx *c) {
   cudaFree(m->diff64);
   cudaFree(m->dDiffOff64);
   cudaFree(m->eamTab);
-  cudaFree(m->redRep);
-  cudaFree(m->redStart);
   delete m;
   c->mixed = nullptr;
 }
@@ -1003,8 +992,8 @@ int sg_mixed_enqueue_reduce(sg_ctx *c, int forceRebuild, bool publish) {
               : m->mixAtoms == 4 * kMixThreads ? k_step_reduce_mixed<4>
               : m->mixAtoms == 2 * kMixThreads ? k_step_reduce_mixed<2>
                                                : k_step_reduce_mixed<1>;
-  MCK(launchK(c->pdl, kern, m->redN, kMixThreads, 0, c->stream,
-      BlockTab{m->redRep, m->redStart, m->redN}, c->rc, c->st, c->pos, c->posLo, c->vel, c->acc, c->fric, m->partDF, m->partF,
+  MCK(launchK(c->pdl, kern, m->redTab.n, kMixThreads, 0, c->stream,
+      m->redTab.view(), c->rc, c->st, c->pos, c->posLo, c->vel, c->acc, c->fric, m->partDF, m->partF,
       c->dRedFirst, m->counter, m->diff64, m->dDiffOff64, c->diffBuf, c->dDiffOff, forceRebuild,
       publish ? PublishArgs{c->hostSt, c->devSeq, c->hostSeq, c->nrep} : PublishArgs{}));
   MCK(cudaGetLastError());
@@ -1075,8 +1064,8 @@ int sg_mixed_enqueue_persistent(sg_ctx *c, int forceRebuild) {
   a.atomTab = c->atomTab.view();
   a.metalTab = c->metalRun.view();
   a.carbonTab = c->carbonTabT.view();
-  a.redTab = BlockTab{m->redRep, m->redStart, m->redN};
-  a.tileRep = c->tileTab.rep;
+  a.redTab = m->redTab.view();
+  a.tileRep = c->tileReps();
   a.tileStart = c->tileTab.start;
   a.tileFirst = c->dTileFirst;
   a.nScanBlocks = c->nScanBlocks;

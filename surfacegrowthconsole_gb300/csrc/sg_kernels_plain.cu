@@ -46,12 +46,11 @@ __global__ void k_integrate_first(BlockTab tab, const RepConst *__restrict__ rc,
                                   int forceRebuild, int *__restrict__ bucket, int cap,
                                   int *__restrict__ blockCount) {
   pdlEnter();
-  const int rep = tab.rep[blockIdx.x];
+  const int rep = tabRep(tab, blockIdx.x);
   const RepConst &P = rc[rep];
   RepState *S = st + rep;
-  const int g = tab.start[blockIdx.x] + threadIdx.x;
-  const int end = P.atomOff + P.nMol;
-  if (g >= end) return;
+  const int g = tabStart(tab, blockIdx.x) + threadIdx.x;
+  if (g >= tabStop(tab, blockIdx.x)) return;
   const int local = g - P.atomOff;
   const int sc = S->stepCount + 1;
   float4 r = pos[g];
@@ -199,7 +198,7 @@ __global__ void __launch_bounds__(128, 8) k_force_both(BlockTab metal, BlockTab 
                                                        float *__restrict__ fric, int rowStride) {
   pdlEnter();
   if ((int)blockIdx.x < metal.nblocks)
-    forceMetalBody<kMT>(blockIdx.x, rc[metal.rep[blockIdx.x]], metal, pos, acc, nn, nbl, posF, Fv, fric, rowStride);
+    forceMetalBody<kMT>(blockIdx.x, rc[tabRep(metal, blockIdx.x)], metal, pos, acc, nn, nbl, posF, Fv, fric, rowStride);
   else
     carbonBody(blockIdx.x - metal.nblocks, carbon, rc, pos, acc, nn, nbl, ns, sl, nrl, rl, rowStride);
 }
@@ -356,19 +355,19 @@ __global__ void __launch_bounds__(kRedThreads) k_cmvel(BlockTab tab, const RepCo
                                                        float *__restrict__ partial,
                                                        const int *__restrict__ redFirst) {
   pdlEnter();
-  const int rep = tab.rep[blockIdx.x];
+  const int rep = tabRep(tab, blockIdx.x);
   const RepConst &P = rc[rep];
   RepState *S = st + rep;
-  const int b = tab.start[blockIdx.x];  // local reduction block index
+  const int g0 = tabStart(tab, blockIdx.x), stop = tabStop(tab, blockIdx.x);
   const int t = threadIdx.x;
   const float h = 0.5f * P.deltaT;
   float e[2][3];
 #pragma unroll
   for (int half = 0; half < 2; half++) {
-    const int local = kRedElems * b + half * kRedThreads + t;
-    if (local < P.nMolMe) {
-      const float4 v = vel[P.atomOff + local];
-      const float4 a = acc[P.atomOff + local];
+    const int g = g0 + half * kRedThreads + t;
+    if (g < stop) {
+      const float4 v = vel[g];
+      const float4 a = acc[g];
       e[half][0] = v.x + h * a.x;
       e[half][1] = v.y + h * a.y;
       e[half][2] = v.z + h * a.z;
@@ -384,7 +383,9 @@ __global__ void __launch_bounds__(kRedThreads) k_cmvel(BlockTab tab, const RepCo
   float *part = partial + (size_t)redFirst[rep] * 3;
   const int nMetalBlocks = (P.nMolMe + kRedElems - 1) / kRedElems;
   if (t == 0) {
-    part[3 * b + 0] = x[0]; part[3 * b + 1] = x[1]; part[3 * b + 2] = x[2];
+    // the blocks' slots are in the order of the table
+    float *own = partial + (size_t)blockIdx.x * 3;
+    own[0] = x[0]; own[1] = x[1]; own[2] = x[2];
     __threadfence();
     const unsigned prev = atomicAdd(&S->cmvCounter, 1u);
     last = (prev == (unsigned)nMetalBlocks - 1);
@@ -457,25 +458,24 @@ __global__ void __launch_bounds__(kRedThreads) k_step_reduce(
     float *__restrict__ partial, const int *__restrict__ redFirst, float *__restrict__ diffBuf,
     const size_t *__restrict__ diffOff, int forceRebuild, PublishArgs pub) {
   pdlEnter();
-  const int rep = tab.rep[blockIdx.x];
+  const int rep = tabRep(tab, blockIdx.x);
   const RepConst &P = rc[rep];
   RepState *S = st + rep;
-  const int b = tab.start[blockIdx.x];
+  const int g0 = tabStart(tab, blockIdx.x), stop = tabStop(tab, blockIdx.x);
   const int t = threadIdx.x;
   const float h = 0.5f * P.deltaT;
   const float cmVelX = (P.nMolMe != 0) ? S->cmVel[0] / (float)P.nMolMe : 0.f;
   float e0[kNumRed], e1[kNumRed];
 #pragma unroll
   for (int half = 0; half < 2; half++) {
-    const int local = kRedElems * b + half * kRedThreads + t;
+    const int g = g0 + half * kRedThreads + t, local = g - P.atomOff;
     float4 r = make_float4(0.f, 0.f, 0.f, 0.f), v = r;
     float frc = 0.f;
-    if (local < P.nMol) {
-      const int g = P.atomOff + local;
+    if (g < stop) {
       r = pos[g];
       v = vel[g];
+      const float4 a = acc[g];
       if (!isFrozen(P, local, r.x, r.y)) {
-        const float4 a = acc[g];
         v.x = v.x + h * a.x;
         v.y = v.y + h * a.y;
         v.z = v.z + h * a.z;
@@ -510,7 +510,7 @@ __global__ void __launch_bounds__(kRedThreads) k_step_reduce(
   float *part = partial + (size_t)redFirst[rep] * kNumRed;
   if (t == 0) {
 #pragma unroll
-    for (int s = 0; s < kNumRed; s++) part[kNumRed * b + s] = x[s];
+    for (int s = 0; s < kNumRed; s++) partial[(size_t)blockIdx.x * kNumRed + s] = x[s];  // slots in the table's order
     __threadfence();
     const unsigned prev = atomicAdd(&S->redCounter, 1u);
     last = (prev == (unsigned)P.nRedBlocks - 1);

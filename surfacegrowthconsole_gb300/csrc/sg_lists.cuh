@@ -53,7 +53,7 @@ __device__ __forceinline__ void scanRankBody(int t, const int *__restrict__ tile
   __shared__ int ws[kWarps], wp[kWarps], wl[kWarps], wh[kWarps], wOcc[kWarps], wOver[kWarps];
   __shared__ int sEx[CELLS + 1];  // exclusive prefix of the block's cell counts
   __shared__ int sBaseL, sBaseH, sBase, sOver;
-  const int rep = tileRep[t / kSub];
+  const int rep = tileRep ? tileRep[t / kSub] : 0;  // no table: one replica
   RepState *S = st + rep;
   if (!rebuilding(S, forceRebuild)) return;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -280,7 +280,7 @@ __device__ __forceinline__ bool nebrNextItem(int *work, int nLight, int nHeavy, 
   } else {
     gc = active[descending ? nHeavy + nLight - 1 - idx : idx - nHeavy];
   }
-  it.rep = tileRep[gc / kCellTile];
+  it.rep = tileRep ? tileRep[gc / kCellTile] : 0;
   const RepConst &P = rc[it.rep];
   const int c = gc - P.cellOff;
   const int hb = cellStart[gc], he = cellStart[gc + 1];

@@ -30,8 +30,6 @@ namespace {
 constexpr size_t kScratchBytes = SG_NOALLOC_SCRATCH_BYTES;
 constexpr int kBs = 128;
 // table capacity: the metal pass has the smallest blocks (kMetalPerBlock atoms)
-constexpr int kMaxTabBlocks = (SG_NOALLOC_MAX_ATOMS + kMetalPerBlock - 1) / kMetalPerBlock;
-constexpr int kMaxTiles = SG_NOALLOC_MAX_CELLS / kCellTile;
 // home atoms per work item of the list build: 4, so that a small system's warps have little to do in
 // sequence (a call on 2,217 / 15,883 atoms: 54.8 / 67.2 us; 8 as in the step, 56.7 / 67.7)
 constexpr int kItem = kMinItemAtoms;
@@ -46,7 +44,7 @@ static __device__ __align__(256) unsigned char g_scratch[kScratchBytes];
 
 // Carving of the scratch array (offsets in bytes, each 256-byte aligned).
 struct Carve {
-  size_t rc, st, tabRep, tabStart, tileRep, cellStart;
+  size_t rc, st, cellStart;
   size_t cellOf, sortIdx, nn, ns, sl, sortPos, rho, posF, Fv, fric, nbl, nrl, rl, active, heavy, work, total;
 };
 constexpr size_t up(size_t x) { return (x + 255) & ~size_t(255); }
@@ -56,9 +54,6 @@ constexpr Carve carve() {
   const size_t N = SG_NOALLOC_MAX_ATOMS;
   c.rc = o; o += up(sizeof(RepConst));
   c.st = o; o += up(sizeof(RepState));
-  c.tabRep = o; o += up(3 * kMaxTabBlocks * sizeof(int));    // atom, metal, carbon tables
-  c.tabStart = o; o += up(3 * kMaxTabBlocks * sizeof(int));
-  c.tileRep = o; o += up(kMaxTiles * sizeof(int));
   c.cellStart = o; o += up(SG_NOALLOC_MAX_CELLS * sizeof(int));
   c.cellOf = o; o += up(N * sizeof(int));
   c.sortIdx = o; o += up(N * sizeof(int));
@@ -97,8 +92,7 @@ std::mutex g_mu;
 // has, up to a multiple of four).
 constexpr int kNoCell = 1 << 30;
 __global__ void __launch_bounds__(kSortThreads) k_noalloc_setup(const __grid_constant__ RepConst P, RepState *st,
-                                                                RepConst *rc, int *tabRep, int *tabStart, int *tileRep,
-                                                                int *work, const float4 *__restrict__ pos,
+                                                                RepConst *rc, int *work, const float4 *__restrict__ pos,
                                                                 int *__restrict__ cellOf, int *__restrict__ nn,
                                                                 int *__restrict__ ns, int *__restrict__ nrl) {
   asm volatile("griddepcontrol.launch_dependents;");  // the sort's few blocks may take their places now
@@ -119,13 +113,6 @@ __global__ void __launch_bounds__(kSortThreads) k_noalloc_setup(const __grid_con
     reinterpret_cast<int *>(rc)[q] = reinterpret_cast<const int *>(&P)[q];
   for (int q = t; q < (int)(sizeof(RepState) / 4); q += n)
     reinterpret_cast<int *>(st)[q] = q == (int)(offsetof(RepState, nebrNow) / 4) ? 1 : 0;
-  for (int b = t; b < 3 * kMaxTabBlocks; b += n) {
-    const int e = b % kMaxTabBlocks;
-    tabRep[b] = 0;
-    // atoms, 128 per block; metal atoms; carbon atoms
-    tabStart[b] = b < kMaxTabBlocks ? e * kBs : b < 2 * kMaxTabBlocks ? e * kMetalPerBlock : P.nMolMe + e * kCarbonPerBlock;
-  }
-  if (t < kMaxTiles) tileRep[t] = 0;
   if (t < 4) work[t] = 0;
 }
 
@@ -311,8 +298,7 @@ extern "C" int sg_compute_forces_noalloc(const sg_simparams *p, sg_float4 *d_pos
   const Carve &K = kCarve;
   RepConst *rc = (RepConst *)(base + K.rc);
   RepState *st = (RepState *)(base + K.st);
-  int *tabRep = (int *)(base + K.tabRep), *tabStart = (int *)(base + K.tabStart);
-  int *tileRep = (int *)(base + K.tileRep), *cellStart = (int *)(base + K.cellStart);
+  int *cellStart = (int *)(base + K.cellStart);
   int *cellOf = (int *)(base + K.cellOf), *sortIdx = (int *)(base + K.sortIdx), *nn = (int *)(base + K.nn), *ns = (int *)(base + K.ns);
   int *sl = (int *)(base + K.sl);
   float4 *sortPos = (float4 *)(base + K.sortPos);
@@ -329,16 +315,16 @@ extern "C" int sg_compute_forces_noalloc(const sg_simparams *p, sg_float4 *d_pos
   const int N = p->nMol;
   const int nMetalBlk = (p->nMolMe + kMetalPerBlock - 1) / kMetalPerBlock;
   const int nCarbBlk = (N - p->nMolMe + kCarbonPerBlock - 1) / kCarbonPerBlock;
-  BlockTab metalTab{tabRep + kMaxTabBlocks, tabStart + kMaxTabBlocks, nMetalBlk};
-  BlockTab carbTab{tabRep + 2 * kMaxTabBlocks, tabStart + 2 * kMaxTabBlocks, nCarbBlk};
+  const BlockTab metalTab{nullptr, nullptr, nMetalBlk, nullptr, 0, kMetalPerBlock, p->nMolMe};
+  const BlockTab carbTab{nullptr, nullptr, nCarbBlk, nullptr, p->nMolMe, kCarbonPerBlock, N};
   const int rowStride = (p->iNebrMax + 3) & ~3;
   const size_t sortSmem = 2 * sizeof(unsigned) * N;
 
-  k_noalloc_setup<<<1 + (N + kSortThreads + 3) / kSortThreads, kSortThreads, 0, s>>>(P, st, rc, tabRep, tabStart, tileRep, work,
+  k_noalloc_setup<<<1 + (N + kSortThreads + 3) / kSortThreads, kSortThreads, 0, s>>>(P, st, rc, work,
                                                                                      pos, cellOf, nn, ns, nrl);
   launchK(true, k_noalloc_sort, P.ncells / kSortCells + 1, kSortThreads, sortSmem, s, N, P.ncells, st, pos, cellOf, cellStart,
           (int)p->blockSize, heavy, active, work, sortIdx, sortPos);
-  launchK(true, k_build_nebr, kBuildBlocks, kNebrWarps * 32, 0, s, tileRep, active, heavy, work, rc, st, cellStart, sortPos, nn,
+  launchK(true, k_build_nebr, kBuildBlocks, kNebrWarps * 32, 0, s, nullptr, active, heavy, work, rc, st, cellStart, sortPos, nn,
           nbl, ns, sl, nrl, rl, rowStride, p->iNebrMax, 0, nullptr, 0);
   if (nMetalBlk)
     launchK(true, k_rho, nMetalBlk, kBs, 0, s, metalTab, rc, pos, nn, nbl, rho, posF, Fv, rowStride);
