@@ -98,6 +98,7 @@ struct sg_ctx {
   int anyMetal = 0, anyCarbon = 0, maxHist = 0;
   // graphs keyed by variant bits (with G_FROM_HOST: upload from hostGraphBufs, step, publish)
   std::map<int, cudaGraphExec_t> graphs;
+  std::map<int, int> singleSteps;  // steps launched one by one, by variant
   HostBufs hostGraphBufs;
   // host mirror of the schedule
   int stepCount = 0;

@@ -956,31 +956,31 @@ int sg_mixed_enqueue_integrate(sg_ctx *c, int forceRebuild, const sg_float4 *hos
   return SG_OK;
 }
 
-// The metal chain (density, metal forces) on the side stream beside the carbon pass, joined
-// before the reduction, as in PLAIN; no centre-of-mass-velocity pass.
+// The metal chain (density, metal forces) on the main stream and the carbon pass beside it on the side
+// stream, joined before the reduction, as in PLAIN; no centre-of-mass-velocity pass.
 int sg_mixed_enqueue_forces(sg_ctx *c) {
   MixedBufs *m = static_cast<MixedBufs *>(c->mixed);
-  const bool fork = c->metalRun.n > 0;
+  const bool metal = c->metalRun.n > 0, carbon = c->carbonTabT.n > 0, fork = metal && carbon;
+  cudaStream_t cs = fork ? c->side : c->stream;
   if (fork) {
     MCK(cudaEventRecord(c->evFork, c->stream));
     MCK(cudaStreamWaitEvent(c->side, c->evFork, 0));
+  }
+  if (metal) {
     launchMetalChain_mixed(c->pdl, c->metalLanes, c->metalRun.n, c->eamStaged ? c->numSMs * 4 : 0,
-                           m->stagedSmem, c->side, c->metalRun.view(), c->rc, c->pos, c->acc,
+                           m->stagedSmem, c->stream, c->metalRun.view(), c->rc, c->pos, c->acc,
                            c->nn, c->nbl, c->rho, c->posF, c->Fv, c->fric, c->rowStride, m->eamTab);
-    if (c->opt.phase_timing) cudaEventRecordWithFlags(c->phaseEv[7], c->side, cudaEventRecordExternal);
     MCK(cudaGetLastError());
   }
-  if (c->carbonTabT.n) {
-    MCK(launchCarbon_mixed(c->pdl, c->carbonBlocks, c->carbonTabT.n, c->stream, c->carbonTabT.view(), c->rc, c->pos,
+  if (c->opt.phase_timing) cudaEventRecordWithFlags(c->phaseEv[7], c->stream, cudaEventRecordExternal);
+  if (carbon)
+    MCK(launchCarbon_mixed(c->pdl, c->carbonBlocks, c->carbonTabT.n, cs, c->carbonTabT.view(), c->rc, c->pos,
                            c->acc, c->nn, c->nbl, c->ns, c->sl, c->nrl, c->rl, c->rowStride));
-  }
-  if (c->opt.phase_timing) cudaEventRecordWithFlags(c->phaseEv[3], c->stream, cudaEventRecordExternal);
+  if (c->opt.phase_timing) cudaEventRecordWithFlags(c->phaseEv[3], cs, cudaEventRecordExternal);
   MCK(cudaGetLastError());
   if (fork) {
     MCK(cudaEventRecord(c->evJoin, c->side));
     MCK(cudaStreamWaitEvent(c->stream, c->evJoin, 0));
-  } else if (c->opt.phase_timing) {
-    cudaEventRecordWithFlags(c->phaseEv[7], c->stream, cudaEventRecordExternal);
   }
   return SG_OK;
 }
