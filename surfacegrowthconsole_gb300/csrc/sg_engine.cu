@@ -943,7 +943,7 @@ static int launchStep(sg_ctx *c, int variant, int steps = 1) {
       return rc;
     }
     if (e != cudaSuccess) return sg_fail(SG_ERR_CUDA, "graph capture: %s", cudaGetErrorString(e));
-    if (steps == 1) c->kernelsPerVariant[variant] = countKernels(g);
+    c->kernelsPerVariant[variant] = countKernels(g) / steps;
     cudaGraphExec_t ex;
     e = cudaGraphInstantiate(&ex, g, 0);
     cudaGraphDestroy(g);

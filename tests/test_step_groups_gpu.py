@@ -42,3 +42,16 @@ def test_groups_match_single_steps(mode, rdf, shear_at):
             assert np.array_equal(one.rdf(0), many.rdf(0))
     one.close()
     many.close()
+
+
+def test_kernels_per_step_after_a_group():
+    p, r, v = system(False, 0)
+    a = np.zeros((p.nMol, 3), np.float32)
+    counts = []
+    for steps in (1, 72):  # a single step; 64 single ones and a group of 8 that ends with the publish
+        sim = Simulation(p)
+        sim.set_state(r, v, a)
+        sim.step(steps)
+        counts.append(sim.kernels_per_step())
+        sim.close()
+    assert counts[0] == counts[1] > 0
