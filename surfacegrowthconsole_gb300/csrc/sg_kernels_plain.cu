@@ -309,42 +309,77 @@ __device__ __forceinline__ float combine(int op, float a, float b) {
   return (a > b) ? b : a;
 }
 
-// Tree over 512 per-thread values (after the first level, done in registers), for NV <= 16
-// values per element, in the reference's pairing (x[t] += x[t + s] for s = 256 ... 1).  The
-// values go through shared memory once; warp v then owns value v, its lane l holding the
-// entries t = l + 32 k, k = 0..15, so the strides s >= 32 pair registers of the same lane and
-// the strides 16..1 are shuffles.  Result valid in lane 0 of warp v (returned to thread 0 via
-// shared memory in x[] of thread 0).
+// The reference's tree over 512 values (x[t] += x[t + s] for s = 256 ... 1), by a warp whose lane l holds
+// the entries t = l + 32 k: the strides s >= 32 pair registers of the same lane, the strides 16..1 are
+// shuffles.  Result in lane 0.
+__device__ __forceinline__ float warpTree512(int op, float (&e)[16]) {
+#pragma unroll
+  for (int n = 8; n >= 1; n >>= 1)
+#pragma unroll
+    for (int k = 0; k < n; k++) e[k] = combine(op, e[k], e[k + n]);
+  float y = e[0];
+#pragma unroll
+  for (int s = 16; s >= 1; s >>= 1) y = combine(op, y, __shfl_down_sync(0xffffffffu, y, s));
+  return y;
+}
+// Trees over 512 per-thread values (after the first level, done in registers), for NV <= 16 values per
+// element: the values go through shared memory once, and warp v then owns value v.  Result in lane 0 of
+// warp v.
 template <int NV>
-__device__ __forceinline__ void blockTree512(float (&x)[NV], const int *ops, float (*sh)[kRedThreads]) {
+__device__ __forceinline__ float blockTree512(const float (&x)[NV], const int *ops, float (*sh)[kRedThreads]) {
   const int t = threadIdx.x;
   const int w = t >> 5, l = t & 31;
 #pragma unroll
   for (int v = 0; v < NV; v++) sh[v][t] = x[v];
   __syncthreads();
-  __shared__ float res[16];
-  if (w < NV) {
+  if (w >= NV) return 0.f;
+  float e[16];
+#pragma unroll
+  for (int k = 0; k < 16; k++) e[k] = sh[w][l + 32 * k];
+  return warpTree512(ops[w], e);
+}
+// The reference's tree over a replica's n block sums, a row of NV values each, zero past them.  Result in
+// lane 0 of warp v for value v.  Up to 128 rows (131,072 atoms) the warp takes its value straight from the
+// rows, one, two or four a lane; the strides past them add zeros (once: x + 0 settles a negative zero, and
+// the reference's extremes include the padding).  More rows go through shared memory as the atoms do.  PLAIN
+// step with both reductions in this form: 2,217 atoms 25.7 -> 25.1 us, 64 replicas 292.7 -> 279.3 (fewer
+// registers and barriers); sixteen rows a lane for every n cost 45,546 atoms 1.1 us.
+template <int K> __device__ __forceinline__ float fewRows(const float *__restrict__ column, int stride, int n, int op) {
+  const int l = threadIdx.x & 31;
+  float e[K];
+#pragma unroll
+  for (int k = 0; k < K; k++) e[k] = combine(op, l + 32 * k < n ? __ldcg(column + stride * (l + 32 * k)) : 0.f, 0.f);
+#pragma unroll
+  for (int m = K / 2; m >= 1; m >>= 1)
+#pragma unroll
+    for (int k = 0; k < m; k++) e[k] = combine(op, e[k], e[k + m]);
+  float y = e[0];
+#pragma unroll
+  for (int s = 16; s >= 1; s >>= 1) y = combine(op, y, __shfl_down_sync(0xffffffffu, y, s));
+  return y;
+}
+template <int NV>
+__device__ __forceinline__ float rowTree(const float *__restrict__ part, int n, const int *ops, float (*sh)[kRedThreads]) {
+  const int t = threadIdx.x, w = t >> 5;
+  if (n <= 128) {
+    if (w >= NV) return 0.f;
     const int op = ops[w];
-    float e[16];
-#pragma unroll
-    for (int k = 0; k < 16; k++) e[k] = sh[w][l + 32 * k];
-#pragma unroll
-    for (int k = 0; k < 8; k++) e[k] = combine(op, e[k], e[k + 8]);  // s = 256
-#pragma unroll
-    for (int k = 0; k < 4; k++) e[k] = combine(op, e[k], e[k + 4]);  // s = 128
-#pragma unroll
-    for (int k = 0; k < 2; k++) e[k] = combine(op, e[k], e[k + 2]);  // s = 64
-    float y = combine(op, e[0], e[1]);                              // s = 32
-#pragma unroll
-    for (int s = 16; s >= 1; s >>= 1) y = combine(op, y, __shfl_down_sync(0xffffffffu, y, s));
-    if (l == 0) res[w] = y;
+    return n <= 32 ? fewRows<1>(part + w, NV, n, op) : n <= 64 ? fewRows<2>(part + w, NV, n, op) : fewRows<4>(part + w, NV, n, op);
   }
-  __syncthreads();
-  if (t == 0) {
+  float carry = 0.f;
+  for (int base = 0; base < n; base += kRedElems) {
+    float x[NV];
 #pragma unroll
-    for (int v = 0; v < NV; v++) x[v] = res[v];
+    for (int s = 0; s < NV; s++) {
+      const float lo = (base + t < n) ? __ldcg(part + NV * (base + t) + s) : 0.f;
+      const float hi = (base + kRedThreads + t < n) ? __ldcg(part + NV * (base + kRedThreads + t) + s) : 0.f;
+      x[s] = combine(ops[s], lo, hi);
+    }
+    __syncthreads();
+    const float y = blockTree512<NV>(x, ops, sh);
+    if (w < NV) carry = base == 0 ? y : combine(ops[w], carry, y);
   }
-  __syncthreads();
+  return carry;
 }
 
 // Centre-of-mass velocity of the metal (ComputeCmVelK, cu:1560-1638) on the velocities after
@@ -378,53 +413,31 @@ __global__ void __launch_bounds__(kRedThreads) k_cmvel(BlockTab tab, const RepCo
   float x[3] = {e[0][0] + e[1][0], e[0][1] + e[1][1], e[0][2] + e[1][2]};
   __shared__ float sh[3][kRedThreads];
   const int ops[3] = {0, 0, 0};
-  blockTree512<3>(x, ops, sh);
+  const float y = blockTree512<3>(x, ops, sh);
+  const int w = t >> 5;
+  const bool owner = w < 3 && (t & 31) == 0;  // holds value w
   __shared__ bool last;
   const int nMetalBlocks = (P.nMolMe + kRedElems - 1) / kRedElems;
   if (nMetalBlocks == 1) {
     // no other block to wait for (a fence, a counter and reading the sums back are 1.9 us of a step: 27.9 ->
-    // 26.0 us with 201 metal atoms); + 0: the
-    // reference's further levels add zeros
-    if (t == 0)
-      for (int c = 0; c < 3; c++) S->cmVel[c] = x[c] + 0.f;
+    // 26.0 us with 201 metal atoms); + 0: the reference's further levels add zeros
+    if (owner) S->cmVel[w] = y + 0.f;
     return;
   }
-  float *part = partial + (size_t)redFirst[rep] * 3;
+  if (owner) partial[(size_t)blockIdx.x * 3 + w] = y;  // the blocks' slots are in the order of the table
+  __syncthreads();
   if (t == 0) {
-    // the blocks' slots are in the order of the table
-    float *own = partial + (size_t)blockIdx.x * 3;
-    own[0] = x[0]; own[1] = x[1]; own[2] = x[2];
     __threadfence();
-    const unsigned prev = atomicAdd(&S->cmvCounter, 1u);
-    last = (prev == (unsigned)nMetalBlocks - 1);
+    last = atomicAdd(&S->cmvCounter, 1u) == (unsigned)nMetalBlocks - 1;
   }
   __syncthreads();
   if (!last) return;
   __threadfence();
   // final tree over the block partials (slots beyond the metal blocks are zero, as the
   // reference's non-metal blocks contribute zero sums)
-  float y[3] = {0.f, 0.f, 0.f};
-  float carry[3] = {0.f, 0.f, 0.f};
-  for (int base = 0; base < nMetalBlocks; base += kRedElems) {
-    float lo[3], hi[3];
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-      lo[c] = (base + t < nMetalBlocks) ? __ldcg(part + 3 * (base + t) + c) : 0.f;
-      hi[c] = (base + kRedThreads + t < nMetalBlocks) ? __ldcg(part + 3 * (base + kRedThreads + t) + c) : 0.f;
-      y[c] = lo[c] + hi[c];
-    }
-    __syncthreads();
-    blockTree512<3>(y, ops, sh);
-    if (t == 0) {
-#pragma unroll
-      for (int c = 0; c < 3; c++) carry[c] = (base == 0) ? y[c] : carry[c] + y[c];
-    }
-    __syncthreads();
-  }
-  if (t == 0) {
-    S->cmVel[0] = carry[0]; S->cmVel[1] = carry[1]; S->cmVel[2] = carry[2];
-    S->cmvCounter = 0;
-  }
+  const float sum = rowTree<3>(partial + (size_t)redFirst[rep] * 3, nMetalBlocks, ops, sh);
+  if (owner) S->cmVel[w] = sum;
+  if (t == 0) S->cmvCounter = 0;
 }
 
 // Per-element values of the step reduction for local atom index `local`.
@@ -513,40 +526,22 @@ __global__ void __launch_bounds__(kRedThreads) k_step_reduce(
     for (int i = t; i < (int)(sizeof(RepState) / 4); i += kRedThreads) sd[i] = __ldcg(ss + i);
   }
   __shared__ float sh[kNumRed][kRedThreads];
-  blockTree512<kNumRed>(x, ops, sh);
+  const float y = blockTree512<kNumRed>(x, ops, sh);
+  const int w = t >> 5;
+  const bool owner = w < kNumRed && (t & 31) == 0;  // holds value w
   __shared__ bool last;
-  float *part = partial + (size_t)redFirst[rep] * kNumRed;
+  if (owner) partial[(size_t)blockIdx.x * kNumRed + w] = y;  // slots in the table's order
+  __syncthreads();
   if (t == 0) {
-#pragma unroll
-    for (int s = 0; s < kNumRed; s++) partial[(size_t)blockIdx.x * kNumRed + s] = x[s];  // slots in the table's order
     __threadfence();
-    const unsigned prev = atomicAdd(&S->redCounter, 1u);
-    last = (prev == (unsigned)P.nRedBlocks - 1);
+    last = atomicAdd(&S->redCounter, 1u) == (unsigned)P.nRedBlocks - 1;
   }
   __syncthreads();
   if (!last) return;
   __threadfence();
-  float y[kNumRed], carry[kNumRed];
-  for (int base = 0; base < P.nRedBlocks; base += kRedElems) {
-#pragma unroll
-    for (int s = 0; s < kNumRed; s++) {
-      const float lo = (base + t < P.nRedBlocks) ? __ldcg(part + kNumRed * (base + t) + s) : 0.f;
-      const float hi = (base + kRedThreads + t < P.nRedBlocks) ? __ldcg(part + kNumRed * (base + kRedThreads + t) + s) : 0.f;
-      y[s] = combine(ops[s], lo, hi);
-    }
-    __syncthreads();
-    blockTree512<kNumRed>(y, ops, sh);
-    if (t == 0) {
-#pragma unroll
-      for (int s = 0; s < kNumRed; s++) carry[s] = (base == 0) ? y[s] : combine(ops[s], carry[s], y[s]);
-    }
-    __syncthreads();
-  }
+  const float sum = rowTree<kNumRed>(partial + (size_t)redFirst[rep] * kNumRed, P.nRedBlocks, ops, sh);
   __shared__ float red[kNumRed];
-  if (t == 0) {
-#pragma unroll
-    for (int s = 0; s < kNumRed; s++) red[s] = carry[s];
-  }
+  if (owner) red[w] = sum;
   __syncthreads();
   float redv[kNumRed];
 #pragma unroll
