@@ -1495,6 +1495,8 @@ int timeSteps(sg_ctx *c, int steps, float *msPerStep) {
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
+  // every trial with its steps in groups, as a long run has them (the first of the two runs captures them)
+  for (int v = 0; v <= (V_SHEAR | V_RDF | V_RDF_ZERO); v++) c->singleSteps[v] = kGroupAfter;
   int rc = sg_step_async(c, 3);
   if (!rc) rc = checkFlags(c);
   float best = 0.f;
