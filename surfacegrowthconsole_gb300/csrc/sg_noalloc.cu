@@ -6,7 +6,7 @@
 // grow the process's device footprint per call.  sg_compute_forces_noalloc serves them: the
 // caller passes device buffers for the inputs and outputs, and every intermediate of the
 // evaluation (cell counts and starts, sorted atoms, neighbour lists, EAM densities, the
-// parameter block, the block tables) lives in one file-scope static device array of
+// parameter block) lives in one file-scope static device array of
 // SG_NOALLOC_SCRATCH_BYTES, which every GPU that loads the library holds until the process
 // exits.
 //
@@ -29,7 +29,6 @@ namespace {
 
 constexpr size_t kScratchBytes = SG_NOALLOC_SCRATCH_BYTES;
 constexpr int kBs = 128;
-// table capacity: the metal pass has the smallest blocks (kMetalPerBlock atoms)
 // home atoms per work item of the list build: 4, so that a small system's warps have little to do in
 // sequence (a call on 2,217 / 15,883 atoms: 54.8 / 67.2 us; 8 as in the step, 56.7 / 67.7)
 constexpr int kItem = kMinItemAtoms;
@@ -86,9 +85,8 @@ constexpr int kMaxDevices = 64;
 unsigned char *g_base[kMaxDevices] = {};
 std::mutex g_mu;
 
-// Block 0 writes the parameter block, clears the state block and the list build's counters, and fills
-// the block tables of a single system: everything that must start fresh on every call.  The others
-// find the cells of kSortThreads atoms each (-1: outside the grid; past the last atom one that no cell
+// Block 0 writes the parameter block and clears the state block and the list build's counters: what must
+// start fresh on every call.  The others find the cells of kSortThreads atoms each (-1: outside the grid; past the last atom one that no cell
 // has, up to a multiple of four).
 constexpr int kNoCell = 1 << 30;
 __global__ void __launch_bounds__(kSortThreads) k_noalloc_setup(const __grid_constant__ RepConst P, RepState *st,
