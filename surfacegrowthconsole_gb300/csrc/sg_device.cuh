@@ -133,7 +133,8 @@ struct RepState {
   int flags;                        // sticky error bits (SG_ERR_* as 1 << code)
   int maxNeighbours, maxCellOcc, nebrOverflow, cellRange, cellOverflow, rdfRange, shortStale;
   int timeouts;                     // bounded device-side waits that gave up (persistent step)
-  int pad[3];
+  unsigned readCounter;             // last-block counter of a download that applies a rescale
+  int pad[2];
 };
 
 // Relevant-list entry of a carbon atom: the neighbour's index relative to its replica's first

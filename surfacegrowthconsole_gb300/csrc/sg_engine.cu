@@ -692,12 +692,12 @@ extern "C" int sg_get_state(sg_ctx *c, int rep, sg_float4 *r, sg_float3 *v, sg_f
     sg_populate(v, (size_t)n * sizeof(*v));
     sg_populate(a, (size_t)n * sizeof(*a));
     BlockTab tab = c->atomTab.view();
-    if (rep >= 0) {  // the replica's entries: the table lists the replicas in order
+    if (rep >= 0 && !v) {  // the replica's entries (the table lists the replicas in order)
       int first = 0;
       for (int q = 0; q < rep; q++) first += (c->hrc[q].nMol + 127) / 128;
       tab = BlockTab{tab.rep + first, tab.start + first, (n + 127) / 128};
     }
-    k_read_state<<<tab.nblocks, 128, 0, c->stream>>>(tab, c->rc, c->st, c->pos, c->vel, c->acc, off,
+    k_read_state<<<tab.nblocks, 128, 0, c->stream>>>(tab, c->rc, c->st, c->pos, c->vel, c->acc, off, n,
                                                      reinterpret_cast<float4 *>(r), reinterpret_cast<float *>(v),
                                                      reinterpret_cast<float *>(a));
     CK(cudaGetLastError());

@@ -69,8 +69,8 @@ __global__ void k_publish_state(const int *src, int *dst, int nwords, unsigned *
                                 unsigned *done);
 __global__ void k_unpack_state(const float4 *sr, const float *sv, const float *sa, float4 *pos, float4 *vel,
                                float4 *acc, float4 *posLo, int n, RepState *st, int nrep);
-__global__ void k_read_state(BlockTab tab, const RepConst *rc, const RepState *st, const float4 *pos, const float4 *vel,
-                             const float4 *acc, int off, float4 *hr, float *hv, float *ha);
+__global__ void k_read_state(BlockTab tab, const RepConst *rc, RepState *st, const float4 *pos, float4 *vel,
+                             const float4 *acc, int off, int count, float4 *hr, float *hv, float *ha);
 __global__ void k_pack3(const float4 *src, float *dst, int n);
 
 }  // namespace sg

@@ -978,38 +978,49 @@ __global__ void k_apply_pending(BlockTab tab, const RepConst *__restrict__ rc, R
 }
 
 // A state download in one launch, straight into the host's arrays (any of hr, hv, ha null: skipped)
-// through the host's page tables: entries [0, tab.nblocks) of the table from `first` on, atom g at
-// g - off of the arrays.  A pending thermostat rescale is applied to the velocities on their way; it
-// stays pending on the device, where the next step's integrator applies the same product.  Rows of
-// three floats go through shared memory so that a warp writes contiguous words.
-__global__ void __launch_bounds__(128) k_read_state(BlockTab tab, const RepConst *__restrict__ rc,
-                                                    const RepState *__restrict__ st, const float4 *__restrict__ pos,
-                                                    const float4 *__restrict__ vel, const float4 *__restrict__ acc, int off,
+// through the host's page tables: the table's atoms in [off, off + count), atom g at g - off of the
+// arrays.  With velocities, a pending thermostat rescale is applied first, as k_apply_pending and
+// k_clear_pending do, to every replica of the table, in place: what the caller has been given is what
+// the context goes on with, whatever is uploaded next.  A replica's rescale is cleared by the last of
+// its blocks to have read it, which costs the many downloads without one nothing.  Rows of three floats
+// go through shared memory so that a warp writes contiguous words.
+__global__ void __launch_bounds__(128) k_read_state(BlockTab tab, const RepConst *__restrict__ rc, RepState *st,
+                                                    const float4 *__restrict__ pos, float4 *__restrict__ vel,
+                                                    const float4 *__restrict__ acc, int off, int count,
                                                     float4 *__restrict__ hr, float *__restrict__ hv, float *__restrict__ ha) {
   __shared__ float sV[3 * 128], sA[3 * 128];
   const int rep = tab.rep[blockIdx.x], t = threadIdx.x;
   const RepConst &P = rc[rep];
-  const RepState *S = st + rep;
+  RepState *S = st + rep;
   const int g0 = tab.start[blockIdx.x], n = min(128, P.atomOff + P.nMol - g0), g = g0 + t;
+  const bool wanted = g0 >= off && g0 < off + count;  // whole blocks: the range is one of replicas
+  const bool pending = hv && S->thermoPending;
+  if (!wanted && !pending) return;
   if (t < n) {
-    if (hr) hr[g - off] = pos[g];
+    if (hr && wanted) hr[g - off] = pos[g];
     if (hv) {
       float4 v = vel[g];
-      if (S->thermoPending) {
+      if (pending) {
         const bool metal = g - P.atomOff < P.nMolMe;
         if (!metal || S->thermoMetal) {
           const float b = metal ? S->betaM : S->betaC;
           v.x = b * v.x; v.y = b * v.y; v.z = b * v.z;
+          vel[g] = v;
         }
       }
       sV[3 * t] = v.x; sV[3 * t + 1] = v.y; sV[3 * t + 2] = v.z;
     }
-    if (ha) {
+    if (ha && wanted) {
       const float4 a = acc[g];
       sA[3 * t] = a.x; sA[3 * t + 1] = a.y; sA[3 * t + 2] = a.z;
     }
   }
   __syncthreads();
+  if (pending && t == 0 && atomicAdd(&S->readCounter, 1u) == (unsigned)(P.nMol + 127) / 128 - 1) {
+    S->thermoPending = 0;
+    S->readCounter = 0;
+  }
+  if (!wanted) return;
   const size_t at = 3 * (size_t)(g0 - off);
 #pragma unroll
   for (int q = 0; q < 3; q++) {
