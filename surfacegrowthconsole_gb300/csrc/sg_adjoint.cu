@@ -1124,7 +1124,8 @@ extern "C" int sg_diff_forces(sg_diff *d, const double *theta, float *out) {
 }
 
 // The reference forces are read in place where the device reads host memory directly (their
-// transfer then overlaps the passes: only the paired atoms' are needed early), else copied first.
+// transfer then overlaps the passes: only the paired atoms' are needed early), else, or at an address
+// that is no multiple of four, copied first.
 extern "C" int sg_diff_force_matching(sg_diff *d, const double *theta, const float *ref, double *loss,
                                       double *grad) {
   if (!d || !theta || !ref) return sg_fail(SG_ERR_INVALID, "sg_diff_force_matching: null argument");
@@ -1132,7 +1133,7 @@ extern "C" int sg_diff_force_matching(sg_diff *d, const double *theta, const flo
   if (int rc = uploadModel(d, theta)) return rc;
   const double inv3N = 1.0 / (3.0 * d->n);
   const float *src = ref;
-  if (!c->hostDirect) {
+  if (!c->hostDirect || (reinterpret_cast<uintptr_t>(ref) & 3) != 0) {
     DCK(cudaMemcpyAsync(c->stage, ref, sizeof(float) * 3 * d->n, cudaMemcpyHostToDevice, c->stream));
     src = c->stage;
   }

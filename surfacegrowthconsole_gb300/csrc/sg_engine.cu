@@ -609,6 +609,13 @@ void sg_populate(void *p, size_t bytes) {
   errno = keep;
 }
 
+// Whether kernels can read and write a state's host rows in place (r as float4 rows, v and a word by
+// word); rows at other addresses, views into a byte buffer, say, can only be copied.
+static bool rowsAligned(const void *r, const void *v, const void *a) {
+  return reinterpret_cast<uintptr_t>(r) % 16 == 0 && reinterpret_cast<uintptr_t>(v) % 4 == 0 &&
+         reinterpret_cast<uintptr_t>(a) % 4 == 0;
+}
+
 // The device address of a host array the GPU can read in place (page-locked, mapped into the
 // unified address space: cudaMallocHost, cudaHostAlloc, cudaHostRegister), else nullptr.
 static const void *mappedHost(const void *h) {
@@ -632,19 +639,13 @@ static const void *mappedHost(const void *h) {
 static int enqueueSetState(sg_ctx *c, int rep, const sg_float4 *r, const sg_float3 *v, const sg_float3 *a) {
   int off, n, rc;
   if ((rc = repRange(c, rep, off, n))) return rc;
-  const float4 *sr;
-  const float *sv, *sa;
-  if (c->hostDirect) {
-    // read in place through the host's page tables; r as float4 rows only when 16-byte aligned
-    // (else copied first), v and a row by row at any 4-byte alignment
-    sr = (reinterpret_cast<uintptr_t>(r) & 15) == 0 ? reinterpret_cast<const float4 *>(r) : nullptr;
-    sv = reinterpret_cast<const float *>(v);
-    sa = reinterpret_cast<const float *>(a);
-  } else {
-    sr = static_cast<const float4 *>(mappedHost(r));
-    sv = static_cast<const float *>(mappedHost(v));
-    sa = static_cast<const float *>(mappedHost(a));
-  }
+  // read in place: any host memory through the host's page tables, else mapped memory; r as float4
+  // rows only when 16-byte aligned, v and a row by row at any 4-byte alignment (else copied first)
+  auto inPlace = [&](const void *h, uintptr_t align) {
+    return reinterpret_cast<uintptr_t>(h) % align ? nullptr : c->hostDirect ? h : mappedHost(h);
+  };
+  const float4 *sr = static_cast<const float4 *>(inPlace(r, 16));
+  const float *sv = static_cast<const float *>(inPlace(v, 4)), *sa = static_cast<const float *>(inPlace(a, 4));
   if (r && !sr) CK(cudaMemcpyAsync(c->pos + off, r, (size_t)n * sizeof(float4), cudaMemcpyHostToDevice, c->stream));
   if (v && !sv) {
     CK(cudaMemcpyAsync(c->stage, v, (size_t)n * 3 * sizeof(float), cudaMemcpyHostToDevice, c->stream));
@@ -684,7 +685,7 @@ extern "C" int sg_get_state(sg_ctx *c, int rep, sg_float4 *r, sg_float3 *v, sg_f
   if (!c) return sg_fail(SG_ERR_INVALID, "null context");
   int off, n, rc;
   if ((rc = repRange(c, rep, off, n))) return rc;
-  if (c->hostDirect && (reinterpret_cast<uintptr_t>(r) & 15) == 0) {
+  if (c->hostDirect && rowsAligned(r, v, a)) {
     // one launch writes the caller's arrays in place, whatever their allocation, and one wait (the
     // route below is six operations and up to three waits: 45,546 atoms into fresh pages 110 us, 72 here)
     if (!r && !v && !a) return SG_OK;
@@ -1120,8 +1121,7 @@ extern "C" int sg_step_from_host(sg_ctx *c, int rep, const sg_float4 *r, const s
   if (!c || (t && (thermo_rep < 0 || thermo_rep >= c->nrep)) || nsteps < 0)
     return sg_fail(SG_ERR_INVALID, "sg_step_from_host: bad arguments");
   int rc;
-  if (nsteps == 1 && c->hostDirect && c->opt.use_graphs && !c->persistent && r && v && a &&
-      (reinterpret_cast<uintptr_t>(r) & 15) == 0) {
+  if (nsteps == 1 && c->hostDirect && c->opt.use_graphs && !c->persistent && r && v && a && rowsAligned(r, v, a)) {
     int off, n;
     if ((rc = repRange(c, rep, off, n))) return rc;
     const int variant = stepVariant(c);
