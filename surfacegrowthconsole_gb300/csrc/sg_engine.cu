@@ -23,6 +23,7 @@
 #include <cstring>
 #include <map>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "sg_api.h"
@@ -592,21 +593,27 @@ static int download3(sg_ctx *c, const float4 *d, sg_float3 *h, int n) {
   return SG_OK;
 }
 
-// The pages of a host array about to be written by the device, made present.  A page that the process
-// has not touched yet costs the device about 19 us to fault in (64 KB; 716,263 atoms' state, 28 MB,
-// took 7.5 to 8.6 ms), the process 2 us, and a present one next to nothing (5 us for 1.8 MB).  Below
-// 128 KB allocators hand out memory in use.  A kernel or mapping that cannot do it leaves it to the
-// device.
-void sg_populate(void *p, size_t bytes) {
+// The pages of a host array about to be written, made present: 1, or 0 where the system cannot tell
+// (memory mapped by a driver, no memory at all, a Linux before 5.14), or -1 if the array cannot be
+// written.  A page that the process has not touched yet costs the device about 19 us to fault in (64 KB;
+// 716,263 atoms' state, 28 MB, took 7.5 to 8.6 ms), the process 2 us, and a present one next to nothing
+// (5 us for 1.8 MB).  A kernel writes only to pages known to be there: what a copy or the process would
+// report as an error, a kernel's write to a read-only page raises as a fault of the device.
+int sg_populate(void *p, size_t bytes) {
 #ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_READ 22
 #define MADV_POPULATE_WRITE 23
 #endif
-  if (!p || bytes < (128u << 10)) return;
+  if (!p || bytes == 0) return 1;
   const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), a = reinterpret_cast<uintptr_t>(p) & ~(page - 1);
+  const size_t len = (reinterpret_cast<uintptr_t>(p) + bytes - a + page - 1) & ~(page - 1);
+  void *at = reinterpret_cast<void *>(a);
   const int keep = errno;
-  (void)madvise(reinterpret_cast<void *>(a), (reinterpret_cast<uintptr_t>(p) + bytes - a + page - 1) & ~(page - 1),
-                MADV_POPULATE_WRITE);
+  int known = 1;
+  if (madvise(at, len, MADV_POPULATE_WRITE) != 0)
+    known = errno == EFAULT || madvise(at, len, MADV_POPULATE_READ) == 0 ? -1 : 0;
   errno = keep;
+  return known;
 }
 
 // Whether kernels can read and write a state's host rows in place (r as float4 rows, v and a word by
@@ -685,13 +692,17 @@ extern "C" int sg_get_state(sg_ctx *c, int rep, sg_float4 *r, sg_float3 *v, sg_f
   if (!c) return sg_fail(SG_ERR_INVALID, "null context");
   int off, n, rc;
   if ((rc = repRange(c, rep, off, n))) return rc;
-  if (c->hostDirect && rowsAligned(r, v, a)) {
+  bool direct = c->hostDirect && rowsAligned(r, v, a);
+  const std::pair<void *, size_t> outs[3] = {{r, n * sizeof(*r)}, {v, n * sizeof(*v)}, {a, n * sizeof(*a)}};
+  for (auto &[p, bytes] : outs) {
+    const int known = sg_populate(p, bytes);
+    if (known < 0) return sg_fail(SG_ERR_INVALID, "sg_get_state: an output array is not writable memory");
+    direct = direct && (known || mappedHost(p));
+  }
+  if (direct) {
     // one launch writes the caller's arrays in place, whatever their allocation, and one wait (the
     // route below is six operations and up to three waits: 45,546 atoms into fresh pages 110 us, 72 here)
     if (!r && !v && !a) return SG_OK;
-    sg_populate(r, (size_t)n * sizeof(*r));
-    sg_populate(v, (size_t)n * sizeof(*v));
-    sg_populate(a, (size_t)n * sizeof(*a));
     BlockTab tab = c->atomTab.view();
     if (rep >= 0 && !v) {  // the replica's entries (the table lists the replicas in order)
       int first = 0;
