@@ -450,9 +450,10 @@ __device__ __forceinline__ float refSquares(const float *__restrict__ ref, int n
       // floats f .. f + 3 belong to atoms a and a + 1, split at atom a + 1's first float
       const long long f = min(4 * (q + u * stride), n3 - 1);
       const int a = (int)(f / 3), cut = (int)(3LL * (a + 1) - f);  // 1..3 floats of atom a
-      const float wa = paired[a] ? 0.f : 1.f, wb = (a + 1 < n && !paired[a + 1]) ? 1.f : 0.f;
-      s += wa * (v[u].x * v[u].x) + (cut > 1 ? wa : wb) * (v[u].y * v[u].y) + (cut > 2 ? wa : wb) * (v[u].z * v[u].z) +
-           wb * (v[u].w * v[u].w);
+      // selected, not weighted with 0 and 1: a square may be infinite
+      const bool wa = !paired[a], wb = a + 1 < n && !paired[a + 1];
+      s += (wa ? v[u].x * v[u].x : 0.f) + ((cut > 1 ? wa : wb) ? v[u].y * v[u].y : 0.f) +
+           ((cut > 2 ? wa : wb) ? v[u].z * v[u].z : 0.f) + (wb ? v[u].w * v[u].w : 0.f);
     }
   }
   for (long long f = 4 * n4 + (long long)b * blockDim.x + threadIdx.x; f < n3; f += stride)
