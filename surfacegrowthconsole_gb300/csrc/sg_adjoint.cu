@@ -138,11 +138,14 @@ __global__ void k_diff_slots(BlockTab tab, const RepConst *__restrict__ rc, cons
 }
 // A warp per atom: its row packed to metal entries of higher slots, the other metal entries and
 // carbon entries, with their numbers in seg[slot] (all metal, carbon, metal of higher slots);
-// paired[atom] set for every metal atom in the grid and for a carbon atom of any LJ pair.
+// paired[atom] set for every metal atom in the grid and for a carbon atom of any LJ pair.  oneSided:
+// rows that did not hold all their entries, of which a pair may be in one only; every metal entry then
+// counts as one of a higher slot (k_diff_sums takes each for its own side).
 __global__ void __launch_bounds__(kDT) k_diff_pack(BlockTab tab, const RepConst *__restrict__ rc,
                                                    const float4 *__restrict__ pos, const int *__restrict__ nn,
                                                    const int *__restrict__ slotOf, int *__restrict__ nbl, int rowStride,
-                                                   int4 *__restrict__ seg, unsigned char *__restrict__ paired) {
+                                                   int4 *__restrict__ seg, unsigned char *__restrict__ paired,
+                                                   bool oneSided) {
   extern __shared__ int sRow[];
   const unsigned full = 0xffffffffu;
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -188,7 +191,7 @@ __global__ void __launch_bounds__(kDT) k_diff_pack(BlockTab tab, const RepConst 
   for (int q = lane; q < nl; q += 32) row[nh + q] = rest[q];
   for (int q = lane; q < nc; q += 32) row[nh + nl + q] = rest[rowStride - 1 - q];
   if (lane == 0) {
-    seg[own] = make_int4(nh + nl, nc, nh, 0);
+    seg[own] = make_int4(nh + nl, nc, oneSided ? nh + nl : nh, 0);
     if (metal) paired[i] = 1;
   }
 }
@@ -659,8 +662,9 @@ __global__ void __launch_bounds__(kPassThreads, kPassBlocks) k_diff_along(const 
 //   energy: phi B(r), f (F'_i + F'_j) B(r)
 //   loss (LOSS; the adjoint of sum e . dE/dr): phi w B'(r), f (F''_i g_i + F''_j g_j) B(r) +
 //   (F'_i + F'_j) w B'(r).
+// ONE_SIDED: a side's terms of each entry, half of phi's and atom i's F' and F'' g.
 constexpr int kSumLoads = 4;  // pairs a thread loads together
-template <bool LOSS>
+template <bool LOSS, bool ONE_SIDED>
 __global__ void __launch_bounds__(kDT) k_diff_sums(const DiffModel *__restrict__ model, DiffPairs pr, int nPairs,
                                                    const float2 *__restrict__ emb, double *__restrict__ grad) {
   __shared__ __align__(16) DiffModel m;
@@ -687,7 +691,7 @@ __global__ void __launch_bounds__(kDT) k_diff_sums(const DiffModel *__restrict__
     for (int q = 0; q < kSumLoads; q++)
       if (p0 + q * stride < nPairs) {
         a[q] = emb[k[q].x];
-        b[q] = emb[k[q].y];
+        b[q] = ONE_SIDED ? make_float2(0.f, 0.f) : emb[k[q].y];
         if (LOSS) w[q] = pr.w[at[q]];
       }
 #pragma unroll
@@ -697,9 +701,9 @@ __global__ void __launch_bounds__(kDT) k_diff_sums(const DiffModel *__restrict__
       const float t = fmaf(r[q] - m.knot[i].x, m.invH, m.knot[i].y), Fd = a[q].x + b[q].x;
       if (LOSS) {
         const float wh = w[q] * m.invH;
-        addPair<false, true>(S, i, t, 0.f, wh, a[q].y + b[q].y, Fd * wh);
+        addPair<false, true>(S, i, t, 0.f, ONE_SIDED ? 0.5f * wh : wh, a[q].y + b[q].y, Fd * wh);
       } else {
-        addPair<true, false>(S, i, t, 1.f, 0.f, Fd, 0.f);
+        addPair<true, false>(S, i, t, ONE_SIDED ? 0.5f : 1.f, 0.f, Fd, 0.f);
       }
     }
   }
@@ -720,7 +724,8 @@ struct DiffGrids {
       : rho(mostBlocks(k_diff_rho<false>, kPassThreads, sms)), energy(mostBlocks(k_diff_rho<true>, kPassThreads, sms)),
         residual(mostBlocks(k_diff_force<true>, kPassThreads, sms)), force(mostBlocks(k_diff_force<false>, kPassThreads, sms)),
         along(mostBlocks(k_diff_along<true>, kPassThreads, sms)), lj(mostBlocks(k_diff_along<false>, kPassThreads, sms)),
-        lossSums(mostBlocks(k_diff_sums<true>, kDT, sms)), energySums(mostBlocks(k_diff_sums<false>, kDT, sms)) {}
+        lossSums(mostBlocks(k_diff_sums<true, false>, kDT, sms)),
+        energySums(mostBlocks(k_diff_sums<false, false>, kDT, sms)) {}
 };
 
 }  // namespace sg
@@ -734,6 +739,7 @@ struct sg_diff {
   explicit sg_diff(int sms) : most(sms) {}
   double r0 = 0, h = 0;  // first knot and interval width of the splines
   bool listed = false;                          // has work lists (of positions, or of none yet)
+  bool oneSided = false;                        // rows were truncated: a pair may be in one of two only
   void *arena = nullptr, *pairArena = nullptr, *pinned = nullptr;  // what the arrays below lie in
   int *slotOf = nullptr;                        // slot of each atom
   unsigned char *paired = nullptr;              // per atom: has a slot in a work list
@@ -819,9 +825,10 @@ struct Carver {
 };
 
 // The packed rows, work lists and pairs of the positions and lists of d's context (built: it has
-// lists).
-static int packLists(sg_diff *d, bool built) {
+// lists; truncated: not all of them whole).
+static int packLists(sg_diff *d, bool built, bool truncated) {
   sg_ctx *c = d->ctx;
+  d->oneSided = truncated;
   DCK(cudaMemsetAsync(d->paired, 0, d->n, c->stream));
   DCK(cudaMemsetAsync(d->counts, 0, 2 * sizeof(int), c->stream));
   DCK(cudaMemsetAsync(d->totals, 0, 2 * sizeof(unsigned long long), c->stream));
@@ -834,7 +841,7 @@ static int packLists(sg_diff *d, bool built) {
     if (smem > 48 * 1024)
       DCK(cudaFuncSetAttribute(k_diff_pack, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     k_diff_pack<<<c->atomTab.n * (128 / warps), 32 * warps, smem, c->stream>>>(
-        c->atomTab.view(), c->rc, c->pos, c->nn, d->slotOf, c->nbl, c->rowStride, d->seg, d->paired);
+        c->atomTab.view(), c->rc, c->pos, c->nn, d->slotOf, c->nbl, c->rowStride, d->seg, d->paired, truncated);
   }
   k_diff_lists<<<c->atomTab.n, 128, 0, c->stream>>>(c->atomTab.view(), c->rc, c->cellStart, c->sortIdx, d->slotOf, built,
                                                     d->paired, d->seg, d->metal, d->carbon, d->counts);
@@ -967,7 +974,7 @@ extern "C" int sg_diff_set_positions(sg_diff *d, const sg_float4 *r) {
   if (int rc = sg_set_state(d->ctx, -1, r, nullptr, nullptr)) return rc;
   const int built = sg_build_lists(d->ctx);  // a list that overflowed is used truncated
   const std::string why = built ? sg_last_error() : "";
-  if (int rc = packLists(d, true)) return rc;
+  if (int rc = packLists(d, true, built != SG_OK)) return rc;
   return built ? sg_fail(built, "%s", why.c_str()) : SG_OK;
 }
 
@@ -1023,7 +1030,7 @@ extern "C" int sg_diff_init_theta(const sg_simparams *pp, double *theta) {
 // the page-locked copy is free again.)
 static int uploadModel(sg_diff *d, const double *theta) {
   if (!d->listed)  // no positions yet: every metal atom without a pair
-    if (int rc = packLists(d, false)) return rc;
+    if (int rc = packLists(d, false, false)) return rc;
   DiffModel &m = *d->hostModel;
   m.r0 = (float)d->r0;
   m.invH = (float)(1.0 / d->h);
@@ -1087,7 +1094,7 @@ static int parameterSums(sg_diff *d) {
     DCK(launchK(true, k_diff_along<LOSS>, std::min(slicesOf(d->nMetal), LOSS ? d->most.along : d->most.lj), kPassThreads, 0,
                 c->stream, d->model, d->metal, d->metalSlices, d->nMetal, d->pairs, d->resid, d->emb, d->out));
   if (d->nOnce)
-    DCK(launchK(true, k_diff_sums<LOSS>, std::min((d->nOnce + kDT - 1) / kDT, LOSS ? d->most.lossSums : d->most.energySums),
+    DCK(launchK(true, d->oneSided ? k_diff_sums<LOSS, true> : k_diff_sums<LOSS, false>, std::min((d->nOnce + kDT - 1) / kDT, LOSS ? d->most.lossSums : d->most.energySums),
                 kDT, 0, c->stream, d->model, d->pairs, d->nOnce, d->emb, d->out));
   return SG_OK;
 }
