@@ -144,8 +144,8 @@ __global__ void k_diff_slots(BlockTab tab, const RepConst *__restrict__ rc, cons
 __global__ void __launch_bounds__(kDT) k_diff_pack(BlockTab tab, const RepConst *__restrict__ rc,
                                                    const float4 *__restrict__ pos, const int *__restrict__ nn,
                                                    const int *__restrict__ slotOf, int *__restrict__ nbl, int rowStride,
-                                                   int4 *__restrict__ seg, unsigned char *__restrict__ paired,
-                                                   bool oneSided) {
+                                                   int restStride, int4 *__restrict__ seg,
+                                                   unsigned char *__restrict__ paired, bool oneSided) {
   extern __shared__ int sRow[];
   const unsigned full = 0xffffffffu;
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -156,8 +156,8 @@ __global__ void __launch_bounds__(kDT) k_diff_pack(BlockTab tab, const RepConst 
   const int metalEnd = P.atomOff + P.nMolMe, own = slotOf[i];
   const bool metal = i < metalEnd;
   // what does not go to the front of the row: lower metal entries from the start, carbon from the
-  // end (backwards); together at most the row
-  int *rest = sRow + w * rowStride;
+  // end (backwards); together at most the row's entries
+  int *rest = sRow + w * restStride;
   const float4 A = pos[i];
   int *row = nbl + (size_t)i * rowStride;
   const int len = nn[i];
@@ -182,14 +182,14 @@ __global__ void __launch_bounds__(kDT) k_diff_pack(BlockTab tab, const RepConst 
     // every lane has read its entry of this and all earlier words: the packed row ends before them
     if (e && slot > own) row[nh + __popc(bh & lower)] = slot;
     else if (e) rest[nl + __popc(bl & lower)] = slot;
-    else if (c) rest[rowStride - 1 - nc - __popc(bc & lower)] = slot;
+    else if (c) rest[restStride - 1 - nc - __popc(bc & lower)] = slot;
     nh += __popc(bh);
     nl += __popc(bl);
     nc += __popc(bc);
     __syncwarp();
   }
   for (int q = lane; q < nl; q += 32) row[nh + q] = rest[q];
-  for (int q = lane; q < nc; q += 32) row[nh + nl + q] = rest[rowStride - 1 - q];
+  for (int q = lane; q < nc; q += 32) row[nh + nl + q] = rest[restStride - 1 - q];
   if (lane == 0) {
     seg[own] = make_int4(nh + nl, nc, oneSided ? nh + nl : nh, 0);
     if (metal) paired[i] = 1;
@@ -835,13 +835,27 @@ static int packLists(sg_diff *d, bool built, bool truncated) {
   DCK(cudaMemsetAsync(d->slotOf, 0xff, sizeof(int) * d->n, c->stream));
   if (built) {
     k_diff_slots<<<c->atomTab.n, 128, 0, c->stream>>>(c->atomTab.view(), c->rc, c->cellStart, c->sortIdx, d->slotOf);
-    // a row of carbon entries per warp in shared memory: one warp a block where rows are very long
-    const int warps = c->rowStride <= 3072 ? kDT / 32 : 1;
-    const size_t smem = sizeof(int) * warps * c->rowStride;
+    // a row's entries per warp in shared memory: one warp a block where they are very many.  A row has
+    // fewer than its frame has atoms, and what the longest one has is looked up only where that, too,
+    // is more than a block can hold.
+    constexpr int kMostRest = 227 * 1024 / sizeof(int);
+    int rest = 1;
+    for (const RepConst &P : c->hrc) rest = std::max(rest, std::min(c->rowStride, P.nMol));
+    if (rest > kMostRest) {
+      int longest = 1;
+      for (int f = 0; f < d->nFrames; f++) {
+        RepState S;
+        if (int rc = sg_read_state(c, f, &S)) return rc;
+        longest = std::max(longest, S.maxNeighbours);
+      }
+      rest = std::min(rest, longest);
+    }
+    const int warps = rest <= 3072 ? kDT / 32 : 1;
+    const size_t smem = sizeof(int) * warps * rest;
     if (smem > 48 * 1024)
       DCK(cudaFuncSetAttribute(k_diff_pack, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     k_diff_pack<<<c->atomTab.n * (128 / warps), 32 * warps, smem, c->stream>>>(
-        c->atomTab.view(), c->rc, c->pos, c->nn, d->slotOf, c->nbl, c->rowStride, d->seg, d->paired, truncated);
+        c->atomTab.view(), c->rc, c->pos, c->nn, d->slotOf, c->nbl, c->rowStride, rest, d->seg, d->paired, truncated);
   }
   k_diff_lists<<<c->atomTab.n, 128, 0, c->stream>>>(c->atomTab.view(), c->rc, c->cellStart, c->sortIdx, d->slotOf, built,
                                                     d->paired, d->seg, d->metal, d->carbon, d->counts);
@@ -1094,8 +1108,8 @@ static int parameterSums(sg_diff *d) {
     DCK(launchK(true, k_diff_along<LOSS>, std::min(slicesOf(d->nMetal), LOSS ? d->most.along : d->most.lj), kPassThreads, 0,
                 c->stream, d->model, d->metal, d->metalSlices, d->nMetal, d->pairs, d->resid, d->emb, d->out));
   if (d->nOnce)
-    DCK(launchK(true, d->oneSided ? k_diff_sums<LOSS, true> : k_diff_sums<LOSS, false>, std::min((d->nOnce + kDT - 1) / kDT, LOSS ? d->most.lossSums : d->most.energySums),
-                kDT, 0, c->stream, d->model, d->pairs, d->nOnce, d->emb, d->out));
+    DCK(launchK(true, d->oneSided ? k_diff_sums<LOSS, true> : k_diff_sums<LOSS, false>,
+                std::min((d->nOnce + kDT - 1) / kDT, LOSS ? d->most.lossSums : d->most.energySums), kDT, 0, c->stream, d->model, d->pairs, d->nOnce, d->emb, d->out));
   return SG_OK;
 }
 
