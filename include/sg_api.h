@@ -361,8 +361,10 @@ int sg_compute_forces_noalloc(const sg_simparams *p, sg_float4 *d_pos, sg_float4
  *     + sum over metal-carbon pairs (r < rCutLJ) 4 eps ((sigma/r)^12 - (sigma/r)^6);
  * the graphene bonded terms have no fit parameter and are left out; forces F = -grad_r E.
  * Frames are independent configurations of systems of the same kind (one parameter block per
- * frame; the frames' iNebrMax must agree).  Pair arithmetic in FP32, sums of energies, losses
- * and gradients in FP64 (through atomics: repeated calls agree to about 1e-7 relative).  The force-matching loss over all frames is
+ * frame; the frames' iNebrMax must agree).  Pair arithmetic in FP32; energies, losses and
+ * gradients are sums in FP64 of FP32 sums of a few dozen terms or compensated ones, so that their
+ * error does not grow with the set (through atomics: repeated calls agree to about 1e-7
+ * relative).  The force-matching loss over all frames is
  *   L = (1 / (3 N)) sum_i |F_i(theta) - F_ref,i|^2      (N: atoms of all frames),
  * its gradient comes from the adjoint pass, which recomputes the densities instead of storing
  * them. */

@@ -18,8 +18,10 @@
 // The adjoint kernel recomputes rho_i and g_i (first pass over the neighbours) and then adds
 // these terms (second pass): nothing per pair is stored.
 //
-// Pair arithmetic in FP32 (FMA on), parameter sums in FP32 per thread (a few tens of terms) and
-// block, energies, losses and gradients summed in FP64 across blocks.
+// Pair arithmetic in FP32 (FMA on).  Sums that grow with the set of frames pass to FP64 after a few dozen
+// terms (a thread's spline coefficients, an atom's pairs) or are compensated (LongSum: losses, the LJ
+// parameters), so that their error does not grow with it; energies, losses and gradients are summed in
+// FP64 across blocks.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -109,6 +111,23 @@ __device__ __forceinline__ float warpSumF(float x) {
   for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
   return x;
 }
+__device__ __forceinline__ double warpSumD(double x) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  return x;
+}
+// A thread's FP32 sum of any number of terms, with what each addition rounds off carried into the next
+// (W. Kahan, "Further remarks on reducing truncation errors", 1965): wrong by two roundings whatever
+// their number, where a plain sum's error grows with it and FP64 runs at 1/64 of the rate.  A sum that
+// has left the finite numbers carries nothing.
+struct LongSum {
+  float s = 0.f, c = 0.f;
+  __device__ __forceinline__ void add(float x) {
+    const float y = __fsub_rn(x, c), t = __fadd_rn(s, y);
+    c = fabsf(t) <= 3.4028234664e38f ? __fsub_rn(__fsub_rn(t, s), y) : 0.f;
+    s = t;
+  }
+};
 // ---- pair lists ----------------------------------------------------------------------------
 // Positions are set once for many evaluations of a fit, so everything that follows from them alone
 // is laid out then: which pairs an evaluation needs (a metal atom's metal entries within the EAM
@@ -410,11 +429,12 @@ __global__ void __launch_bounds__(kPassThreads) k_diff_rho(const DiffModel *__re
     if (ENERGY) {
       // the slice's atoms of one frame in one sum; a slice whose atoms are of several adds them singly
       const int rep = __shfl_sync(0xffffffffu, a.rep, 0);
+      const double u = (double)x[1] + (double)F;
       if (__all_sync(0xffffffffu, a.rep < 0 || a.rep == rep)) {
-        const float u = warpSumF(x[1]), Fw = warpSumF(F);
-        if (lane == 0 && rep >= 0) atomicAdd(&energy[rep], (double)u + (double)Fw);
+        const double all = warpSumD(u);
+        if (lane == 0 && rep >= 0) atomicAdd(&energy[rep], all);
       } else if (a.rep >= 0) {
-        atomicAdd(&energy[a.rep], (double)x[1] + (double)F);
+        atomicAdd(&energy[a.rep], u);
       }
     }
   }
@@ -442,7 +462,7 @@ __device__ __forceinline__ float refSquares(const float *__restrict__ ref, int n
   const long long n3 = 3LL * n;
   const bool aligned = (reinterpret_cast<uintptr_t>(ref) & 15) == 0;
   const long long n4 = aligned ? n3 / 4 : 0, stride = (long long)nb * blockDim.x;
-  float s = 0.f;
+  LongSum s;
   for (long long q = (long long)b * blockDim.x + threadIdx.x; q < n4; q += 2 * stride) {
     float4 v[2];
 #pragma unroll
@@ -455,13 +475,13 @@ __device__ __forceinline__ float refSquares(const float *__restrict__ ref, int n
       const int a = (int)(f / 3), cut = (int)(3LL * (a + 1) - f);  // 1..3 floats of atom a
       // selected, not weighted with 0 and 1: a square may be infinite
       const bool wa = !paired[a], wb = a + 1 < n && !paired[a + 1];
-      s += (wa ? v[u].x * v[u].x : 0.f) + ((cut > 1 ? wa : wb) ? v[u].y * v[u].y : 0.f) +
-           ((cut > 2 ? wa : wb) ? v[u].z * v[u].z : 0.f) + (wb ? v[u].w * v[u].w : 0.f);
+      s.add((wa ? v[u].x * v[u].x : 0.f) + ((cut > 1 ? wa : wb) ? v[u].y * v[u].y : 0.f) +
+            ((cut > 2 ? wa : wb) ? v[u].z * v[u].z : 0.f) + (wb ? v[u].w * v[u].w : 0.f));
     }
   }
   for (long long f = 4 * n4 + (long long)b * blockDim.x + threadIdx.x; f < n3; f += stride)
-    if (!paired[f / 3]) s += ref[f] * ref[f];
-  return s;
+    if (!paired[f / 3]) s.add(ref[f] * ref[f]);
+  return s.s;
 }
 __global__ void __launch_bounds__(kDT) k_diff_ref(const float *__restrict__ ref, int n,
                                                   const unsigned char *__restrict__ paired, double *__restrict__ lossPart) {
@@ -499,7 +519,7 @@ __global__ void __launch_bounds__(kPassThreads, kPassBlocks) k_diff_force(const 
   };
   DiffAtom next = atomOf(blockIdx.x);
   loadModel(model, m);
-  float loss = 0.f;
+  LongSum loss;
   for (int slice = blockIdx.x, turn = 0; slice < nSlices; slice += grid, turn++) {
     const DiffAtom a = next;
     next = atomOf(slice + grid);
@@ -532,7 +552,7 @@ __global__ void __launch_bounds__(kPassThreads, kPassBlocks) k_diff_force(const 
         const float4 want = resid[a.slot];
         const float ex = x[0] - want.x, ey = x[1] - want.y, ez = x[2] - want.z;
         resid[a.slot] = make_float4(scale * ex, scale * ey, scale * ez, 0.f);
-        loss += ex * ex + ey * ey + ez * ez;
+        loss.add(ex * ex + ey * ey + ez * ez);
       } else {
         const size_t f = 3 * (size_t)sortIdx[a.slot];
         out[f] = x[0];
@@ -542,8 +562,8 @@ __global__ void __launch_bounds__(kPassThreads, kPassBlocks) k_diff_force(const 
     }
   }
   if (LOSS && threadIdx.x < 32) {
-    loss = warpSumF(loss);
-    if (threadIdx.x == 0) atomicAdd(sumsCopy(sums) + kDP, (double)loss);
+    const float all = warpSumF(loss.s);
+    if (threadIdx.x == 0) atomicAdd(sumsCopy(sums) + kDP, (double)all);
   }
 }
 
@@ -612,10 +632,11 @@ __global__ void __launch_bounds__(kPassThreads, kPassBlocks) k_diff_along(const 
   const int nSlices = (nMetal + 31) / 32;
   DiffAtom next = diffAtom(metal, slices, nMetal, blockIdx.x);
   loadModel(model, m);
-  float ge = 0.f, gs = 0.f;
+  LongSum sumE, sumS;
   for (int slice = blockIdx.x, turn = 0; slice < nSlices; slice += gridDim.x, turn++) {
     const DiffAtom a = next;
     next = diffAtom(metal, slices, nMetal, slice + gridDim.x);
+    float ge = 0.f, gs = 0.f;  // the slice's
     if (LOSS) {
       const float4 Ei = a.slot >= 0 ? resid[a.slot] : make_float4(0.f, 0.f, 0.f, 0.f);
       const float Fdd = a.slot >= 0 ? emb[a.slot].y : 0.f;
@@ -651,8 +672,10 @@ __global__ void __launch_bounds__(kPassThreads, kPassBlocks) k_diff_along(const 
                          gs += 24.f * m.eps * (2.f * s12 - s6) * m.invSig;  // dU / d sigma
                        });
     }
+    sumE.add(ge);
+    sumS.add(gs);
   }
-  const double e = blockSum(ge), q = blockSum(gs);
+  const double e = blockSum(sumE.s), q = blockSum(sumS.s);
   if (threadIdx.x == 0 && e != 0.0) atomicAdd(sumsCopy(sums), e);
   if (threadIdx.x == 0 && q != 0.0) atomicAdd(sumsCopy(sums) + 1, q);
 }
@@ -663,7 +686,8 @@ __global__ void __launch_bounds__(kPassThreads, kPassBlocks) k_diff_along(const 
 //   loss (LOSS; the adjoint of sum e . dE/dr): phi w B'(r), f (F''_i g_i + F''_j g_j) B(r) +
 //   (F'_i + F'_j) w B'(r).
 // ONE_SIDED: a side's terms of each entry, half of phi's and atom i's F' and F'' g.
-constexpr int kSumLoads = 4;  // pairs a thread loads together
+constexpr int kSumLoads = 4;   // pairs a thread loads together
+constexpr int kSumRounds = 8;  // rounds of them (32 pairs) after which the columns pass to the totals
 template <bool LOSS, bool ONE_SIDED>
 __global__ void __launch_bounds__(kDT) k_diff_sums(const DiffModel *__restrict__ model, DiffPairs pr, int nPairs,
                                                    const float2 *__restrict__ emb, double *__restrict__ grad) {
@@ -673,7 +697,8 @@ __global__ void __launch_bounds__(kDT) k_diff_sums(const DiffModel *__restrict__
   loadModel(model, m);
   pdlEnter();
   const int stride = gridDim.x * kDT;
-  for (int p0 = blockIdx.x * kDT + threadIdx.x; p0 < nPairs; p0 += kSumLoads * stride) {
+  for (int b0 = blockIdx.x * kDT, round = 1; b0 < nPairs; b0 += kSumLoads * stride, round++) {
+    const int p0 = b0 + threadIdx.x;
     float r[kSumLoads], w[kSumLoads];
     int at[kSumLoads];
     int2 k[kSumLoads];
@@ -705,6 +730,11 @@ __global__ void __launch_bounds__(kDT) k_diff_sums(const DiffModel *__restrict__
       } else {
         addPair<true, false>(S, i, t, ONE_SIDED ? 0.5f : 1.f, 0.f, Fd, 0.f);
       }
+    }
+    if (round % kSumRounds == 0) {
+      flushSums(S, grad);
+      __syncthreads();
+      clearSums(S);
     }
   }
   flushSums(S, grad);
