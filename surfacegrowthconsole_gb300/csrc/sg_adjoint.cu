@@ -762,6 +762,9 @@ struct DiffGrids {
 
 using namespace sg;
 
+// Most places of pairs laid out at once: they and the threads' strides over them are 32-bit numbers.
+constexpr unsigned long long kMostPlaces = (1ull << 31) - (1ull << 24);
+
 struct sg_diff {
   sg_ctx *ctx = nullptr;
   int nFrames = 0, n = 0;
@@ -781,6 +784,8 @@ struct sg_diff {
   DiffPairs pairs{};
   unsigned long long pairCap = 0, onceCap = 0;  // pairs the arrays hold
   int nOnce = 0;
+  unsigned long long mostPlaces = kMostPlaces;
+  int broken = SG_OK;                           // what the last set of positions failed with: no lists
   float2 *emb = nullptr;                        // per slot: F', then F'' or F'' g
   float4 *resid = nullptr;                      // per slot
   // results on the device and page-locked on the host: the copies of the sums, then the
@@ -903,8 +908,7 @@ static int packLists(sg_diff *d, bool built, bool truncated) {
   DCK(cudaMemcpyAsync(pairs, d->totals, sizeof pairs, cudaMemcpyDeviceToHost, c->stream));
   DCK(cudaStreamSynchronize(c->stream));
   d->nMetal = d->nCarbon = d->nOnce = 0;  // until the pairs are there
-  d->listed = true;
-  if (pairs[0] >= (1ull << 31)) return sg_fail(SG_ERR_NOMEM, "sg_diff: %llu pairs in one set of frames", pairs[0]);
+  if (pairs[0] > d->mostPlaces) return sg_fail(SG_ERR_NOMEM, "sg_diff: %llu pairs in one set of frames", pairs[0]);
   if (pairs[0] > d->pairCap || pairs[1] > d->onceCap) {
     // an eighth more than asked: a later set of positions rarely has as many more
     const unsigned long long all = pairs[0] + pairs[0] / 8 + 1, once = pairs[1] + pairs[1] / 8 + 1;
@@ -940,6 +944,18 @@ static int packLists(sg_diff *d, bool built, bool truncated) {
   if (built && d->nOnce)
     k_diff_once<<<(counts[0] + kDT - 1) / kDT, kDT, 0, c->stream>>>(d->metal, d->metalSlices, counts[0], d->pairs);
   DCK(cudaGetLastError());
+  return SG_OK;
+}
+// The same; without lists, every evaluation returns the error until a set of positions has them again.
+static int setLists(sg_diff *d, bool built, bool truncated) {
+  d->broken = packLists(d, built, truncated);
+  d->listed = d->broken == SG_OK;
+  return d->broken;
+}
+
+// Most places of pairs laid out at once, for the sets of positions to come (0: as many as there can be).
+int sg_diff_limit_places(sg_diff *d, unsigned long long places) {
+  d->mostPlaces = places && places < kMostPlaces ? places : kMostPlaces;
   return SG_OK;
 }
 
@@ -1018,7 +1034,7 @@ extern "C" int sg_diff_set_positions(sg_diff *d, const sg_float4 *r) {
   if (int rc = sg_set_state(d->ctx, -1, r, nullptr, nullptr)) return rc;
   const int built = sg_build_lists(d->ctx);  // a list that overflowed is used truncated
   const std::string why = built ? sg_last_error() : "";
-  if (int rc = packLists(d, true, built != SG_OK)) return rc;
+  if (int rc = setLists(d, true, built != SG_OK)) return rc;
   return built ? sg_fail(built, "%s", why.c_str()) : SG_OK;
 }
 
@@ -1073,8 +1089,9 @@ extern "C" int sg_diff_init_theta(const sg_simparams *pp, double *theta) {
 // theta as the kernels read it, on its way to the device.  (Every call ends with its stream empty, so
 // the page-locked copy is free again.)
 static int uploadModel(sg_diff *d, const double *theta) {
+  if (d->broken) return sg_fail(d->broken, "sg_diff: no pair lists, sg_diff_set_positions failed");
   if (!d->listed)  // no positions yet: every metal atom without a pair
-    if (int rc = packLists(d, false, false)) return rc;
+    if (int rc = setLists(d, false, false)) return rc;
   DiffModel &m = *d->hostModel;
   m.r0 = (float)d->r0;
   m.invH = (float)(1.0 / d->h);

@@ -122,6 +122,7 @@ struct sg_ctx {
 int sg_fail(int code, const char *fmt, ...);
 
 int sg_populate(void *p, size_t bytes);
+int sg_diff_limit_places(struct sg_diff *d, unsigned long long places);
 int sg_make_range_tab(sg_ctx *c, DevTab &t, int bs, int which);
 int sg_read_state(sg_ctx *c, int rep, sg::RepState *out);
 int sg_get_diffusion_print(sg_ctx *c, int rep, float *table, int *nprints);
