@@ -680,6 +680,16 @@ __global__ void __launch_bounds__(kPassThreads, kPassBlocks) k_diff_along(const 
   if (threadIdx.x == 0 && q != 0.0) atomicAdd(sumsCopy(sums) + 1, q);
 }
 
+// w of the metal pairs counted once (pr.w) alone, where the pairs were laid out anew since k_diff_along.
+__global__ void __launch_bounds__(kDT) k_diff_w(DiffPairs pr, int nPairs, const float4 *__restrict__ resid) {
+  for (long long p = (long long)blockIdx.x * kDT + threadIdx.x; p < nPairs; p += (long long)gridDim.x * kDT) {
+    const int2 k = pr.both[p];
+    const int place = pr.place[p];
+    const float4 D = pr.dir[place], Ei = resid[k.x], Ek = resid[k.y];
+    pr.w[place] = D.x * (Ei.x - Ek.x) + D.y * (Ei.y - Ek.y) + D.z * (Ei.z - Ek.z);
+  }
+}
+
 // The spline coefficients' share, a thread per metal pair counted once (its two sides' terms are
 // alike: r and w are the same from both, and only F' and F'' g differ).
 //   energy: phi B(r), f (F'_i + F'_j) B(r)
@@ -762,6 +772,11 @@ struct DiffGrids {
 
 using namespace sg;
 
+// A run of slices whose pairs are laid out together: the first atom (a multiple of 32) and the number of
+// atoms of each work list, and the metal pairs counted once.
+struct DiffBatch {
+  int metal, nMetal, carbon, nCarbon, nOnce;
+};
 // Most places of pairs laid out at once: they and the threads' strides over them are 32-bit numbers.
 constexpr unsigned long long kMostPlaces = (1ull << 31) - (1ull << 24);
 
@@ -778,12 +793,14 @@ struct sg_diff {
   unsigned char *paired = nullptr;              // per atom: has a slot in a work list
   DiffWork *metal = nullptr, *carbon = nullptr;  // the work lists and their slices
   DiffSlice *metalSlices = nullptr, *carbonSlices = nullptr;
-  int *counts = nullptr, nMetal = 0, nCarbon = 0;
+  int *counts = nullptr, nMetal = 0;
   unsigned long long *totals = nullptr;         // places of all pairs, metal pairs counted once
   int4 *seg = nullptr;                          // per slot: its row's segments (k_diff_pack)
   DiffPairs pairs{};
   unsigned long long pairCap = 0, onceCap = 0;  // pairs the arrays hold
-  int nOnce = 0;
+  // One batch of all slices, laid out with the positions; or several, where that is more than memory
+  // holds, that each pass lays out in turn.
+  std::vector<DiffBatch> batches;
   unsigned long long mostPlaces = kMostPlaces;
   int broken = SG_OK;                           // what the last set of positions failed with: no lists
   float2 *emb = nullptr;                        // per slot: F', then F'' or F'' g
@@ -859,9 +876,105 @@ struct Carver {
   }
 };
 
+static void freePairs(sg_diff *d) {
+  cudaFree(d->pairArena);
+  d->pairArena = nullptr;
+  d->pairCap = d->onceCap = 0;
+}
+// Memory for the arrays of so many pairs and metal pairs counted once, in place of what there was.
+static bool pairMemory(sg_diff *d, unsigned long long all, unsigned long long once) {
+  auto lay = [&](Carver v) {
+    v.take(d->pairs.dir, all);
+    v.take(d->pairs.slot, all);
+    v.take(d->pairs.r, all);
+    v.take(d->pairs.w, all);
+    v.take(d->pairs.both, once);
+    v.take(d->pairs.rOnce, once);
+    v.take(d->pairs.place, once);
+    return v.used;
+  };
+  freePairs(d);
+  if (cudaMalloc(&d->pairArena, lay(Carver{nullptr})) != cudaSuccess) {
+    cudaGetLastError();
+    d->pairArena = nullptr;
+    return false;
+  }
+  lay(Carver{static_cast<char *>(d->pairArena)});
+  d->pairCap = all;
+  d->onceCap = once;
+  return true;
+}
+constexpr size_t kPlaceBytes = sizeof(float4) + sizeof(int) + 2 * sizeof(float);   // dir, slot, r, w
+constexpr size_t kOnceBytes = sizeof(int2) + sizeof(float) + sizeof(int);          // both, rOnce, place
+
+// The pairs of a batch into the arrays.
+static int layPairs(sg_diff *d, const DiffBatch &b) {
+  sg_ctx *c = d->ctx;
+  const DiffWork *lists[2] = {d->metal + b.metal, d->carbon + b.carbon};
+  const DiffSlice *slices[2] = {d->metalSlices + b.metal / 32, d->carbonSlices + b.carbon / 32};
+  const int n[2] = {b.nMetal, b.nCarbon};
+  for (int l = 0; l < 2; l++)
+    if (n[l])
+      k_diff_pairs<<<(n[l] + kDT / 32 - 1) / (kDT / 32), kDT, 0, c->stream>>>(lists[l], slices[l], n[l], c->rc, c->sortPos,
+                                                                              c->nbl, c->rowStride, d->pairs);
+  if (b.nOnce) k_diff_once<<<(n[0] + kDT - 1) / kDT, kDT, 0, c->stream>>>(lists[0], slices[0], n[0], d->pairs);
+  DCK(cudaGetLastError());
+  return SG_OK;
+}
+
+// The slices in batches that fit the memory there is (n: the atoms of the two work lists; needed: places
+// of all pairs), each batch's slices numbered from its own first place.
+static int splitPairs(sg_diff *d, const int n[2], unsigned long long needed) {
+  sg_ctx *c = d->ctx;
+  DiffWork *lists[2] = {d->metal, d->carbon};
+  DiffSlice *slices[2] = {d->metalSlices, d->carbonSlices};
+  std::vector<DiffSlice> all((n[0] + 31) / 32 + (n[1] + 31) / 32);  // metal slices first
+  const int metalN = (n[0] + 31) / 32;
+  DCK(cudaMemcpyAsync(all.data(), slices[0], sizeof(DiffSlice) * metalN, cudaMemcpyDeviceToHost, c->stream));
+  DCK(cudaMemcpyAsync(all.data() + metalN, slices[1], sizeof(DiffSlice) * (all.size() - metalN), cudaMemcpyDeviceToHost,
+                      c->stream));
+  DCK(cudaStreamSynchronize(c->stream));
+  auto places = [](const DiffSlice &s) { return 32ull * (s.most + s.mostC); };
+  unsigned long long largest = 1;
+  for (const DiffSlice &s : all) largest = std::max(largest, places(s));
+  freePairs(d);
+  size_t freeBytes = 0, total = 0;
+  DCK(cudaMemGetInfo(&freeBytes, &total));
+  // nine tenths of what is free, and less where that cannot be had in one piece; every place may be of a
+  // metal pair counted once
+  unsigned long long cap = std::min<unsigned long long>(freeBytes / (kPlaceBytes + kOnceBytes) / 10 * 9,
+                                                        std::min(d->mostPlaces, needed));
+  for (; cap >= largest && !pairMemory(d, cap, cap); cap /= 2) {
+  }
+  if (cap < largest) return sg_fail(SG_ERR_NOMEM, "sg_diff: memory for %llu pairs", largest);
+  d->batches.clear();
+  for (size_t s = 0; s < all.size();) {
+    const size_t s0 = s;
+    for (unsigned long long sum = 0; s < all.size() && sum + places(all[s]) <= cap; s++) sum += places(all[s]);
+    const int m0 = 32 * (int)std::min(s0, (size_t)metalN), m1 = std::min(32 * (int)std::min(s, (size_t)metalN), n[0]);
+    const int c0 = 32 * (int)(std::max(s0, (size_t)metalN) - metalN);
+    const int c1 = std::min(32 * (int)(std::max(s, (size_t)metalN) - metalN), n[1]);
+    d->batches.push_back(DiffBatch{m0, std::max(m1 - m0, 0), c0, std::max(c1 - c0, 0), 0});
+  }
+  for (DiffBatch &b : d->batches) {
+    const int at[2] = {b.metal, b.carbon}, count[2] = {b.nMetal, b.nCarbon};
+    DCK(cudaMemsetAsync(d->totals, 0, 2 * sizeof(unsigned long long), c->stream));
+    for (int l = 0; l < 2; l++)
+      if (count[l])
+        k_diff_slices<<<(count[l] + kDT - 1) / kDT, kDT, 0, c->stream>>>(lists[l] + at[l], count[l], slices[l] + at[l] / 32,
+                                                                         d->totals);
+    DCK(cudaGetLastError());
+    unsigned long long pairs[2];
+    DCK(cudaMemcpyAsync(pairs, d->totals, sizeof pairs, cudaMemcpyDeviceToHost, c->stream));
+    DCK(cudaStreamSynchronize(c->stream));
+    b.nOnce = (int)pairs[1];
+  }
+  return d->batches.size() == 1 ? layPairs(d, d->batches[0]) : SG_OK;
+}
+
 // The packed rows, work lists and pairs of the positions and lists of d's context (built: it has
 // lists; truncated: not all of them whole).
-static int packLists(sg_diff *d, bool built, bool truncated) {
+static int packLists(sg_diff *d, bool built, bool truncated) try {
   sg_ctx *c = d->ctx;
   d->oneSided = truncated;
   DCK(cudaMemsetAsync(d->paired, 0, d->n, c->stream));
@@ -907,44 +1020,18 @@ static int packLists(sg_diff *d, bool built, bool truncated) {
   unsigned long long pairs[2];
   DCK(cudaMemcpyAsync(pairs, d->totals, sizeof pairs, cudaMemcpyDeviceToHost, c->stream));
   DCK(cudaStreamSynchronize(c->stream));
-  d->nMetal = d->nCarbon = d->nOnce = 0;  // until the pairs are there
-  if (pairs[0] > d->mostPlaces) return sg_fail(SG_ERR_NOMEM, "sg_diff: %llu pairs in one set of frames", pairs[0]);
-  if (pairs[0] > d->pairCap || pairs[1] > d->onceCap) {
-    // an eighth more than asked: a later set of positions rarely has as many more
-    const unsigned long long all = pairs[0] + pairs[0] / 8 + 1, once = pairs[1] + pairs[1] / 8 + 1;
-    auto lay = [&](Carver v) {
-      v.take(d->pairs.dir, all);
-      v.take(d->pairs.slot, all);
-      v.take(d->pairs.r, all);
-      v.take(d->pairs.w, all);
-      v.take(d->pairs.both, once);
-      v.take(d->pairs.rOnce, once);
-      v.take(d->pairs.place, once);
-      return v.used;
-    };
-    cudaFree(d->pairArena);
-    d->pairArena = nullptr;
-    d->pairCap = d->onceCap = 0;
-    if (cudaMalloc(&d->pairArena, lay(Carver{nullptr})) != cudaSuccess) {
-      cudaGetLastError();
-      d->pairArena = nullptr;
-      return sg_fail(SG_ERR_NOMEM, "sg_diff: memory for %llu pairs", all);
-    }
-    lay(Carver{static_cast<char *>(d->pairArena)});
-    d->pairCap = all;
-    d->onceCap = once;
-  }
-  d->nOnce = (int)pairs[1];
   d->nMetal = counts[0];
-  d->nCarbon = counts[1];
-  for (int l = 0; l < 2; l++)
-    if (built && counts[l])
-      k_diff_pairs<<<(counts[l] + kDT / 32 - 1) / (kDT / 32), kDT, 0, c->stream>>>(
-          lists[l], slices[l], counts[l], c->rc, c->sortPos, c->nbl, c->rowStride, d->pairs);
-  if (built && d->nOnce)
-    k_diff_once<<<(counts[0] + kDT - 1) / kDT, kDT, 0, c->stream>>>(d->metal, d->metalSlices, counts[0], d->pairs);
-  DCK(cudaGetLastError());
-  return SG_OK;
+  if (pairs[0] <= d->mostPlaces) {
+    // an eighth more than asked: a later set of positions rarely has as many more
+    if ((pairs[0] <= d->pairCap && pairs[1] <= d->onceCap) ||
+        pairMemory(d, pairs[0] + pairs[0] / 8 + 1, pairs[1] + pairs[1] / 8 + 1)) {
+      d->batches.assign(1, DiffBatch{0, counts[0], 0, counts[1], (int)pairs[1]});
+      return built ? layPairs(d, d->batches[0]) : SG_OK;
+    }
+  }
+  return splitPairs(d, counts, pairs[0]);
+} catch (const std::bad_alloc &) {
+  return sg_fail(SG_ERR_NOMEM, "sg_diff: host memory for the batches of pairs");
 }
 // The same; without lists, every evaluation returns the error until a set of positions has them again.
 static int setLists(sg_diff *d, bool built, bool truncated) {
@@ -1118,6 +1205,16 @@ static int uploadModel(sg_diff *d, const double *theta) {
 // Slices of a work list of n atoms, a block each.
 static int slicesOf(int n) { return (n + 31) / 32; }
 
+// f(batch) for every batch, its pairs in the arrays.
+template <typename F> static int overBatches(sg_diff *d, F f) {
+  for (const DiffBatch &b : d->batches) {
+    if (d->batches.size() > 1)
+      if (int rc = layPairs(d, b)) return rc;
+    if (int rc = f(b)) return rc;
+  }
+  return SG_OK;
+}
+
 // F'(rho) of the metal atoms, then the forces: packed into `force`, or (ref) the residuals and the
 // loss, with refBlocks blocks for the atoms without a pair (their sums at out + kSums) in the same
 // launch or (own) in one on the side stream.  That one starts when the reference forces of the atoms
@@ -1125,12 +1222,16 @@ static int slicesOf(int n) { return (n + 31) / 32; }
 // most of the transfer (64 frames of 20,432 atoms: 281 us an evaluation instead of 236).
 static int forces(sg_diff *d, float *force, const float *ref, float scale, int refBlocks, bool own) {
   sg_ctx *c = d->ctx;
-  const int nm = slicesOf(d->nMetal);
   // k_diff_rho also clears the sums, so it runs (one block) without metal too
-  const int refGather = ref ? std::min((d->n + kPassThreads - 1) / kPassThreads, c->numSMs * kRefBlocks) : 0;
-  DCK(launchK(false, k_diff_rho<false>, std::max(1, std::min(nm, d->most.rho) + refGather), kPassThreads, 0, c->stream,
-              d->model, d->metal, d->metalSlices, d->nMetal, c->rc, d->pairs.r, d->emb, nullptr, d->out, ref, d->n,
-              d->paired, d->slotOf, d->resid, refGather));
+  int refGather = ref ? std::min((d->n + kPassThreads - 1) / kPassThreads, c->numSMs * kRefBlocks) : 0;
+  int rc = overBatches(d, [&](const DiffBatch &b) {
+    DCK(launchK(false, k_diff_rho<false>, std::max(1, std::min(slicesOf(b.nMetal), d->most.rho) + refGather), kPassThreads, 0,
+                c->stream, d->model, d->metal + b.metal, d->metalSlices + b.metal / 32, b.nMetal, c->rc, d->pairs.r, d->emb,
+                nullptr, d->out, ref, d->n, d->paired, d->slotOf, d->resid, refGather));
+    refGather = 0;  // with the first batch
+    return (int)SG_OK;
+  });
+  if (rc) return rc;
   if (own) {
     DCK(cudaEventRecord(c->evFork, c->stream));
     DCK(cudaStreamWaitEvent(c->side, c->evFork, 0));
@@ -1139,25 +1240,46 @@ static int forces(sg_diff *d, float *force, const float *ref, float scale, int r
     DCK(cudaEventRecord(c->evJoin, c->side));
     refBlocks = 0;
   }
-  const int blocks = std::min(nm + slicesOf(d->nCarbon), ref ? d->most.residual : d->most.force) + refBlocks;
-  if (blocks > 0)
-    DCK(launchK(true, ref ? k_diff_force<true> : k_diff_force<false>, blocks, kPassThreads, 0, c->stream, d->model, d->metal,
-                d->metalSlices, d->nMetal, d->carbon, d->carbonSlices, d->nCarbon, c->sortIdx, d->pairs, d->emb, force, ref,
-                scale, d->resid, d->out, d->out + kSums, d->n, d->paired, refBlocks));
-  return SG_OK;
+  return overBatches(d, [&](const DiffBatch &b) {
+    const int blocks =
+        std::min(slicesOf(b.nMetal) + slicesOf(b.nCarbon), ref ? d->most.residual : d->most.force) + refBlocks;
+    if (blocks > 0)
+      DCK(launchK(true, ref ? k_diff_force<true> : k_diff_force<false>, blocks, kPassThreads, 0, c->stream, d->model,
+                  d->metal + b.metal, d->metalSlices + b.metal / 32, b.nMetal, d->carbon + b.carbon,
+                  d->carbonSlices + b.carbon / 32, b.nCarbon, c->sortIdx, d->pairs, d->emb, force, ref, scale, d->resid,
+                  d->out, d->out + kSums, d->n, d->paired, refBlocks));
+    refBlocks = 0;  // with the first batch
+    return (int)SG_OK;
+  });
 }
 
 // The parameter sums of an energy or loss evaluation, after its densities (and residuals).
 template <bool LOSS>
 static int parameterSums(sg_diff *d) {
   sg_ctx *c = d->ctx;
-  if (d->nMetal)
-    DCK(launchK(true, k_diff_along<LOSS>, std::min(slicesOf(d->nMetal), LOSS ? d->most.along : d->most.lj), kPassThreads, 0,
-                c->stream, d->model, d->metal, d->metalSlices, d->nMetal, d->pairs, d->resid, d->emb, d->out));
-  if (d->nOnce)
-    DCK(launchK(true, d->oneSided ? k_diff_sums<LOSS, true> : k_diff_sums<LOSS, false>,
-                std::min((d->nOnce + kDT - 1) / kDT, LOSS ? d->most.lossSums : d->most.energySums), kDT, 0, c->stream, d->model, d->pairs, d->nOnce, d->emb, d->out));
-  return SG_OK;
+  auto along = [&](const DiffBatch &b) {
+    if (b.nMetal)
+      DCK(launchK(true, k_diff_along<LOSS>, std::min(slicesOf(b.nMetal), LOSS ? d->most.along : d->most.lj), kPassThreads, 0,
+                  c->stream, d->model, d->metal + b.metal, d->metalSlices + b.metal / 32, b.nMetal, d->pairs, d->resid,
+                  d->emb, d->out));
+    return (int)SG_OK;
+  };
+  auto sums = [&](const DiffBatch &b) {
+    const int most = LOSS ? d->most.lossSums : d->most.energySums, blocks = std::min((b.nOnce + kDT - 1) / kDT, most);
+    if (b.nOnce && LOSS && d->batches.size() > 1) k_diff_w<<<blocks, kDT, 0, c->stream>>>(d->pairs, b.nOnce, d->resid);
+    if (b.nOnce)
+      DCK(launchK(true, d->oneSided ? k_diff_sums<LOSS, true> : k_diff_sums<LOSS, false>, blocks, kDT, 0, c->stream, d->model,
+                  d->pairs, b.nOnce, d->emb, d->out));
+    return (int)SG_OK;
+  };
+  if (d->batches.size() == 1 || !LOSS)
+    return overBatches(d, [&](const DiffBatch &b) {
+      const int rc = along(b);
+      return rc ? rc : sums(b);
+    });
+  // the sums need F'' g of both atoms of a pair, which may lie in different batches
+  const int rc = overBatches(d, along);
+  return rc ? rc : overBatches(d, sums);
 }
 
 extern "C" int sg_diff_energy(sg_diff *d, const double *theta, double *energy, double *grad) {
@@ -1167,10 +1289,15 @@ extern "C" int sg_diff_energy(sg_diff *d, const double *theta, double *energy, d
   const size_t bytes = sizeof(double) * (kSums + d->nFrames);
   DCK(cudaMemsetAsync(d->out, 0, bytes, c->stream));
   if (d->nMetal) {
-    DCK(launchK(false, k_diff_rho<true>, std::min(slicesOf(d->nMetal), d->most.energy), kPassThreads, 0, c->stream, d->model, d->metal, d->metalSlices, d->nMetal, c->rc,
-                d->pairs.r, d->emb, d->out + kSums, d->out, nullptr, d->n, d->paired, d->slotOf, d->resid, 0));
-    if (grad)
-      if (int rc = parameterSums<false>(d)) return rc;
+    int rc = overBatches(d, [&](const DiffBatch &b) {
+      if (b.nMetal)
+        DCK(launchK(false, k_diff_rho<true>, std::min(slicesOf(b.nMetal), d->most.energy), kPassThreads, 0, c->stream,
+                    d->model, d->metal + b.metal, d->metalSlices + b.metal / 32, b.nMetal, c->rc, d->pairs.r, d->emb,
+                    d->out + kSums, d->out, nullptr, d->n, d->paired, d->slotOf, d->resid, 0));
+      return (int)SG_OK;
+    });
+    if (!rc && grad) rc = parameterSums<false>(d);
+    if (rc) return rc;
   }
   DCK(cudaMemcpyAsync(d->hostOut, d->out, bytes, cudaMemcpyDeviceToHost, c->stream));
   DCK(cudaStreamSynchronize(c->stream));
