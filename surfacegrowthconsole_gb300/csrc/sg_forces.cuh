@@ -5,6 +5,7 @@
 // including unit defines SG_KN(name) to name its kernels.
 #pragma once
 #include "sg_device.cuh"
+#include "sg_pairmath.h"
 
 #ifndef SG_KN
 #error "define SG_KN(name) before including sg_forces.cuh"
@@ -44,55 +45,6 @@ namespace sg {
 struct EamPair {
   float phi, dphi, df;
 };
-// x^20, and x^20 with x^19, by repeated squaring on error-free float pairs: the square of
-// (h, l) is (h h, fma(h, h, -h h) + 2 h l), three instructions, so both powers come out rounded
-// from about 46 bits (error at most 0.501 ulp over |x| < 2.3; powf documents 4) for a fraction of two
-// powf calls.  The PLAIN metal passes are bound by instruction issue (63-65% of the issue slots);
-// with these and the shared reciprocals below k_force_metal takes 50.8 us instead of 68.7 and
-// k_rho 29.4 instead of 32.0 on bulk Au (55,296 atoms, ncu).
-// The pair functions call them with |x| below 2; past 64 the powers come near the largest float,
-// where the pairs' error terms would turn an infinity into a NaN: powf decides there (and for NaN).
-struct FPair {
-  float h, l;
-};
-__device__ __forceinline__ FPair pairSquare(FPair a) {
-  FPair r;
-  r.h = __fmul_rn(a.h, a.h);
-  r.l = __fmaf_rn(__fadd_rn(a.h, a.h), a.l, __fmaf_rn(a.h, a.h, -r.h));
-  return r;
-}
-// a b rounded to float
-__device__ __forceinline__ float pairProduct(FPair a, FPair b) {
-  const float p = __fmul_rn(a.h, b.h);
-  const float e = __fmaf_rn(a.h, b.l, __fmaf_rn(a.l, b.h, __fmaf_rn(a.h, b.h, -p)));
-  return __fadd_rn(p, e);
-}
-__device__ __forceinline__ float pow20(float x) {
-  if (!(fabsf(x) < 64.f)) return powf(x, 20.f);
-  const FPair x4 = pairSquare(pairSquare(FPair{x, 0.f}));
-  return pairProduct(pairSquare(pairSquare(x4)), x4);
-}
-__device__ __forceinline__ void pow19and20(float x, float &x19, float &x20) {
-  if (!(fabsf(x) < 64.f)) {
-    x19 = powf(x, 19.f);
-    x20 = powf(x, 20.f);
-    return;
-  }
-  const FPair x2 = pairSquare(FPair{x, 0.f}), x4 = pairSquare(x2), x16 = pairSquare(pairSquare(x4));
-  FPair x3;
-  x3.h = __fmul_rn(x2.h, x);
-  x3.l = __fmaf_rn(x2.l, x, __fmaf_rn(x2.h, x, -x3.h));
-  x19 = pairProduct(x16, x3);
-  x20 = pairProduct(x16, x4);
-}
-// a / b with r = 1 / b rounded to nearest: the quotient a r corrected once by its exact remainder
-// is a / b rounded to nearest (P. Markstein, "Computation of elementary functions on the IBM RISC
-// System/6000 processor", 1990), the same bits as the IEEE division.  The pair functions divide by
-// each of two denominators three or four times; one reciprocal serves them all.
-__device__ __forceinline__ float divBy(float a, float b, float r) {
-  const float q = __fmul_rn(a, r);
-  return __fmaf_rn(__fmaf_rn(-b, q, a), r, q);
-}
 __device__ __forceinline__ EamPair eamPair(const RepConst &P, float r) {
   const float x = r * P.rei;
   const float xm1 = x - 1.f;
