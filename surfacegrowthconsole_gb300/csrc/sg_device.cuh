@@ -298,11 +298,13 @@ __device__ __forceinline__ void setFlag(RepState *st, int code) {
 
 // Programmatic dependent launch.  A kernel of the step chain, launched with the
 // programmatic-serialization attribute, is scheduled once every block of its predecessor in the
-// stream has exited (the implicit trigger: no kernel calls launch_dependents, so waiting blocks
-// never hold SM slots the predecessor still needs), overlapping its launch with the
-// predecessor's completion; it waits here, before its first global memory access, for the
-// predecessor grid to complete with its memory visible.  Every kernel of the chain waits, so
-// completion is transitive.  Launched without the attribute, the wait returns at once.
+// stream has exited (the implicit trigger: no kernel of a step calls launch_dependents, so waiting
+// blocks never hold SM slots the predecessor still needs; k_noalloc_setup calls it, for the few blocks
+// of the sort behind it), overlapping its launch with the predecessor's completion; it waits here for
+// the predecessor grid to complete with its memory visible, before its first access to memory that a
+// kernel of the chain writes (k_diff_sums reads the model, copied ahead of the whole chain, before
+// it).  Every kernel of the chain waits, so completion is transitive.  Launched without the attribute,
+// the wait returns at once.
 __device__ __forceinline__ void pdlEnter() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }

@@ -1161,7 +1161,7 @@ extern "C" int sg_get_phase_times(sg_ctx *c, float *ms, int n) {
   if (!c || !c->opt.phase_timing) return -sg_fail(SG_ERR_UNSUPPORTED, "phase_timing is off");
   cudaError_t e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return -sg_fail(SG_ERR_CUDA, "%s", cudaGetErrorString(e));
-  // integrate, rebuild (sort + list build), metal chain (side stream), carbon pass, forces
+  // integrate, rebuild (sort + list build), metal chain, carbon pass (side stream), forces
   // (fork to join), reduce, extra, list build alone
   const int from[8] = {0, 1, 2, 2, 2, 4, 5, 8}, to[8] = {1, 2, 7, 3, 4, 5, 6, 2};
   const int np = 8;

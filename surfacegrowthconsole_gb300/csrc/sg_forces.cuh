@@ -170,7 +170,9 @@ __device__ __forceinline__ void SG_KN(rhoBody)(int e, const RepConst &P, BlockTa
     const int n = nn[i];
     const int *row = nbl + (size_t)i * rowStride;
     // kMetalBatch entries per lane per round: their indices, then their positions, load
-    // together; their densities are added in pairs (fewer roundings in sequence)
+    // together; their densities are added in pairs.  (No more and no less exact than one after the
+    // other: over 80 states of bulk Ni the PLAIN form's NVE drift is (6.2 +- 0.6) 1e-5 eV/atom/ns,
+    // (5.6 +- 0.6) in sequence, (5.8 +- 0.5) in MIXED, and single states scatter by 3e-5 around MIXED's.)
     int k[kMetalBatch];  // the first round's indices leave before n is known
 #pragma unroll
     for (int q = 0; q < kMetalBatch; q++) k[q] = (sub + q * MT < rowStride) ? row[sub + q * MT] : -1;

@@ -851,7 +851,8 @@ int sg_mixed_init(sg_ctx *c) {
       for (int fn = 0; fn < 2; fn++) tab.push_back(hermite(a[2 * fn], a[2 * fn + 1], b[2 * fn], b[2 * fn + 1], h));
     }
   }
-  // replicas of one metal share a table: 32 KB that stay in every L1 instead of 32 KB a replica
+  // replicas of the first replica's metal share its table: 32 KB that stay in every L1 instead of 32 KB a
+  // replica (replicas of other metals keep a table each)
   m->ownTab.resize(c->nrep);
   int firstTab = -1;
   for (int r = 0; r < c->nrep; r++) {
