@@ -610,8 +610,8 @@ int sg_populate(void *p, size_t bytes) {
   void *at = reinterpret_cast<void *>(a);
   const int keep = errno;
   int known = 1;
-  if (madvise(at, len, MADV_POPULATE_WRITE) != 0)
-    known = errno == EFAULT || madvise(at, len, MADV_POPULATE_READ) == 0 ? -1 : 0;
+  if (madvise(at, len, MADV_POPULATE_WRITE) != 0)  // EINVAL: no right to write, a driver's mapping, an old Linux
+    known = errno == EFAULT || (errno == EINVAL && madvise(at, len, MADV_POPULATE_READ) == 0) ? -1 : 0;
   errno = keep;
   return known;
 }
